@@ -42,27 +42,36 @@ __device__ __forceinline__ BinResult bin_f64(const BinGridD& g, const double* ed
     const double z = g.ki[0] * w.x + g.ki[1] * w.y + g.ki[2] * w.z;
     const double n = sqrt(x * x + y * y + z * z);
     if (!(n > 0) || !finite_r(n) || fabs(n - 1) > 512 * Eps<double>::eps) return b;
-    const double mu = z / n, s = hypot(x, y) / n;
+    const DivBy by_n = div_by(n);
+    const double mu = quot(z, by_n), s = quot(hypot(x, y), by_n);
     b.mu = mu;
     if (s <= 256 * Eps<double>::eps) {
         b.pole = mu >= 0 ? 1 : -1;
         b.valid = true;
         return b;
     }
-    const double u = mu >= 0 ? (0.5 * s * s) / (1 + mu) : 1 - (0.5 * s * s) / (1 - mu);
+    const double part = quot(0.5 * s * s, div_by(1 + fabs(mu)));
+    const double u = mu >= 0 ? part : 1 - part;
     if (!(u >= 0 && u <= 1)) return b;
-    uint32_t lo = 0, hi = g.nt;
-    while (lo + 1 < hi) {
-        const uint32_t mid = lo + (hi - lo) / 2;
-        if (u >= edges[mid]) lo = mid;
-        else hi = mid;
-    }
+    // the largest row whose lower edge is at or below u: guessed from the scattering angle as in
+    // bin_f32 and settled against the stored edges (a binary search costs ten dependent loads)
+    const float am = fminf(fabsf((float)mu), 1.f);
+    const float acos_am = sqrtf(1.f - am) *
+        fmaf(fmaf(fmaf(-0.0187293f, am, 0.0742610f), am, -0.2121144f), am, 1.5707288f);
+    const float theta = mu >= 0 ? acos_am : 3.14159265f - acos_am;
+    const int last = (int)g.nt - 1;
+    int row = __float2int_rd(theta * ((float)g.nt * 0.318309886f));
+    row = row < 0 ? 0 : (row > last ? last : row);
+    while (row > 0 && u < edges[row]) --row;
+    while (row < last && u >= edges[row + 1]) ++row;
+    uint32_t lo = (uint32_t)row;
     for (unsigned c = 0; c < 2; ++c) {
         const uint32_t e = lo + c;
         if (e == 0 || e >= g.nt) continue;
+        const double near = 64 * Eps<double>::eps * fmax(fabs(u), fabs(edges[e]));
+        if (!(fabs(u - edges[e]) <= near)) continue;
         const double width = fmin(edges[e] - edges[e - 1], edges[e + 1] - edges[e]);
-        const double tol = fmin(64 * Eps<double>::eps * fmax(fabs(u), fabs(edges[e])), 1e-7 * width);
-        if (fabs(u - edges[e]) <= tol) {
+        if (fabs(u - edges[e]) <= fmin(near, 1e-7 * width)) {
             b.snapped = (u != edges[e]);
             lo = e;
             break;
@@ -70,7 +79,7 @@ __device__ __forceinline__ BinResult bin_f64(const BinGridD& g, const double* ed
     }
     double phi = atan2(y, x);
     if (phi >= kPi) phi -= 2 * kPi;
-    const double v = (phi + kPi) / (2 * kPi);
+    const double v = quot(phi + kPi, DivBy{2 * kPi, 1.0 / (2 * kPi), true});
     double index = v * g.np;
     const double nearest = floor(index + 0.5);
     if (fabs(index - nearest) <= fmin(64 * Eps<double>::eps * g.np, 1e-7)) {

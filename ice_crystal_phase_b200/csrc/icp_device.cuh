@@ -54,28 +54,47 @@ template <class R> __device__ __forceinline__ bool finite_r(R x)
     return x == x && rabs(x) <= (sizeof(R) == 4 ? R(3.4028234663852886e38) : R(1.7976931348623157e308));
 }
 
+// Quotients by one divisor, rounded as the division operator rounds them.  The reciprocal is
+// evaluated once (correctly rounded), and each quotient is refined twice with the exact FMA
+// remainder: Markstein's theorem (IBM J. Res. Dev. 34, 1990) gives the correctly rounded quotient
+// from a correctly rounded reciprocal and a faithful quotient, away from overflow and underflow.
+// Numerators or divisors outside 2^-900 .. 2^900 take the operator (zeros keep their sign).  The
+// operator costs the FP64 trace kernels a divergent call for every zero component and the same
+// reciprocal again for every component of a vector.
+struct DivBy {
+    double b, y;
+    bool ok;
+};
+__device__ __forceinline__ bool mid_range(double x)
+{
+    return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x07b00000u < 0x70800000u;
+}
+__device__ __forceinline__ DivBy div_by(double b) { return {b, __drcp_rn(b), mid_range(b)}; }
+__device__ __forceinline__ double quot(double a, const DivBy& d)
+{
+    const double q0 = a * d.y;
+    const double q1 = fma(fma(-d.b, q0, a), d.y, q0);
+    double q = fma(fma(-d.b, q1, a), d.y, q1);
+    if (!(mid_range(a) && d.ok)) {
+        q = q0;
+        if (!(a == 0 && d.ok)) q = a / d.b;
+    }
+    return q;
+}
+__device__ __forceinline__ V3<double> quot(V3<double> a, const DivBy& d) { return {quot(a.x, d), quot(a.y, d), quot(a.z, d)}; }
+
 // Unit vector.  FP64: the reference's scale-then-normalise (math.hpp:38-47) so that exit
 // directions, and hence bins, follow the reference bit pattern where the inputs agree.
 // FP32: one reciprocal square root.
 __device__ __forceinline__ V3<float> unit(V3<float> a) { return a * rsqrtf(dot(a, a)); }
 __device__ __forceinline__ V3<double> unit(V3<double> a)
 {
-    const double s = fmax(fabs(a.x), fmax(fabs(a.y), fabs(a.z)));
-    a = a / s;
-    const double n = sqrt(dot(a, a));
-    return a / n;
+    a = quot(a, div_by(fmax(fabs(a.x), fmax(fabs(a.y), fabs(a.z)))));
+    return quot(a, div_by(sqrt(dot(a, a))));
 }
 
-// |d x n| as the reference evaluates it (flux_interface.hpp:42-45): scaled by the largest
-// component in FP64 so that the refraction cosine, and the exit direction, round identically.
+// |d x n| (flux_interface.hpp:42-45)
 __device__ __forceinline__ float sine_of(V3<float> s) { return sqrtf(dot(s, s)); }
-__device__ __forceinline__ double sine_of(V3<double> s)
-{
-    const double scale = fmax(fabs(s.x), fmax(fabs(s.y), fabs(s.z)));
-    if (!(scale > 0)) return 0.0;
-    const V3<double> t = s / scale;
-    return scale * sqrt(dot(t, t));
-}
 
 // ---------------------------------------------------------------- counter RNG
 // SplitMix64 finaliser over seed + golden * (3*id + dim + 1) (math.hpp:136-146).
@@ -131,7 +150,7 @@ template <class R> __host__ __device__ inline Media<R> make_media(double ni, dou
 // medium.  `e` is the ray's current frame vector.  The transmitted flux is 1 - R for each of
 // s and p, so power is conserved to one rounding per interface; its Mueller off-diagonal
 // term is sqrt(Ts*Tp) = ts*tp.  Partial reflection and total internal reflection are both
-// evaluated and selected per lane (no divergent branch between them).
+// evaluated and selected per lane (no divergent branch between them).  The binary64 form follows it.
 template <class R>
 __device__ __forceinline__ Interface<R> split(V3<R> d, V3<R> e, Stokes<R> S, V3<R> n, const Media<R>& M)
 {
@@ -167,32 +186,7 @@ __device__ __forceinline__ Interface<R> split(V3<R> d, V3<R> e, Stokes<R> S, V3<
     out.ci = ci;
     const bool tir = st > R(1);
     R Rs, Rp, zr, zi, ct;
-    if constexpr (sizeof(R) == 8) {
-        // reference arithmetic (flux_interface.hpp:59-79)
-        if (tir) {
-            const R inv = R(1) / st;
-            const R beta = st * sqrt_r((R(1) - inv) * (R(1) + inv));
-            R x1 = a * ci, y1 = b * beta, x2 = b * ci, y2 = a * beta;
-            const R s1 = rmax(rabs(x1), rabs(y1)), s2 = rmax(rabs(x2), rabs(y2));
-            x1 /= s1; y1 /= s1; x2 /= s2; y2 /= s2;
-            const R d1 = x1 * x1 + y1 * y1, d2 = x2 * x2 + y2 * y2;
-            const R rsr = (x1 * x1 - y1 * y1) / d1, rsi = (R(-2) * x1 * y1) / d1;
-            const R rpr = (x2 * x2 - y2 * y2) / d2, rpi = (R(-2) * x2 * y2) / d2;
-            Rs = R(1);
-            Rp = R(1);
-            zr = rsr * rpr + rsi * rpi; // rs * conj(rp)
-            zi = rsi * rpr - rsr * rpi;
-            ct = R(0);
-        } else {
-            ct = sqrt_r((R(1) - st) * (R(1) + st));
-            const R ds = a * ci + b * ct, dp = b * ci + a * ct;
-            const R rs = (a * ci - b * ct) / ds, rp = (b * ci - a * ct) / dp;
-            Rs = rs * rs;
-            Rp = rp * rp;
-            zr = rs * rp;
-            zi = R(0);
-        }
-    } else {
+    {
         // binary32: both branches, selected per lane
         const R k2 = (R(1) - st) * (R(1) + st);
         ct = sqrt_r(rmax(k2, R(0)));
@@ -230,6 +224,96 @@ __device__ __forceinline__ Interface<R> split(V3<R> d, V3<R> e, Stokes<R> S, V3<
         out.t = {R(0), R(0), R(0), R(0)};
         out.balance = S.I > R(0) ? rabs(out.r.I - S.I) / S.I : R(0);
     }
+    return out;
+}
+
+// Binary64: the reference's arithmetic, operation for operation (flux_interface.hpp:42-79, with
+// |d x n| scaled by its largest component so that the refraction cosine, and the exit direction,
+// round identically).  What the two kinds of reflection share -- a square root, two reciprocals, two
+// quotients -- is evaluated once with selected operands; only the phase of a total reflection
+// is left to a branch.
+__device__ __forceinline__ Interface<double> split(V3<double> d, V3<double> e, Stokes<double> S, V3<double> n,
+                                                   const Media<double>& M)
+{
+    Interface<double> out;
+    if (M.matched) {
+        out.s = e;
+        out.dt = d;
+        out.t = S;
+        out.dr = unit(d - n * (2.0 * dot(d, n)));
+        out.r = {0.0, 0.0, 0.0, 0.0};
+        out.ci = -dot(d, n);
+        out.has_t = true;
+        out.tir = false;
+        out.balance = 0.0;
+        return out;
+    }
+    double ci = -dot(d, n);
+    ci = rmin(1.0, rmax(0.0, ci));
+    V3<double> s = cross(d, n);
+    const double scale = fmax(fabs(s.x), fmax(fabs(s.y), fabs(s.z)));
+    const V3<double> t = quot(s, div_by(scale));
+    const double len = sqrt(dot(t, t));
+    const double sine = scale > 0 ? scale * len : 0.0;
+    s = quot(t, div_by(len));
+    if (!(sine > 0)) s = e;
+    out.s = s;
+    // Basis rotation (e, d x e) -> (s, d x s): c = e.s, sg = (d x e).s
+    const double c = dot(e, s);
+    const double sg = dot(cross(d, e), s);
+    const double cos2 = c * c - sg * sg, sin2p = 2.0 * c * sg;
+    const double Q = cos2 * S.Q + sin2p * S.U;
+    const double U = -sin2p * S.Q + cos2 * S.U;
+    const double a = M.a, b = M.b;
+    const double st = M.eta * sine;
+    out.dr = unit(d + n * (2.0 * ci));
+    out.ci = ci;
+    const bool tir = st > 1.0;
+    const double inv = __drcp_rn(tir ? st : 2.0);
+    const double root = sqrt(tir ? (1.0 - inv) * (1.0 + inv) : (1.0 - st) * (1.0 + st));
+    const double u = tir ? st * root : root; // beta of a total reflection, else cos of the refracted ray
+    const double aci = a * ci, bci = b * ci, bu = b * u, au = a * u;
+    const DivBy D1 = div_by(tir ? rmax(rabs(aci), rabs(bu)) : aci + bu);
+    const DivBy D2 = div_by(tir ? rmax(rabs(bci), rabs(au)) : bci + au);
+    const double q1 = quot(tir ? aci : aci - bu, D1), q2 = quot(tir ? bci : bci - au, D2);
+    double Rs, Rp, zr, zi;
+    if (tir) {
+        const double x1 = q1, x2 = q2, y1 = quot(bu, D1), y2 = quot(au, D2);
+        const DivBy E1 = div_by(x1 * x1 + y1 * y1), E2 = div_by(x2 * x2 + y2 * y2);
+        const double rsr = quot(x1 * x1 - y1 * y1, E1), rsi = quot(-2.0 * x1 * y1, E1);
+        const double rpr = quot(x2 * x2 - y2 * y2, E2), rpi = quot(-2.0 * x2 * y2, E2);
+        Rs = 1.0;
+        Rp = 1.0;
+        zr = rsr * rpr + rsi * rpi; // rs * conj(rp)
+        zi = rsi * rpr - rsr * rpi;
+    } else {
+        Rs = q1 * q1;
+        Rp = q2 * q2;
+        zr = q1 * q2;
+        zi = 0.0;
+    }
+    out.tir = tir;
+    out.has_t = !tir;
+    const double hs = 0.5 * (Rs + Rp), hd = 0.5 * (Rs - Rp);
+    out.r.I = hs * S.I + hd * Q;
+    out.r.Q = hd * S.I + hs * Q;
+    out.r.U = zr * U - zi * S.V;
+    out.r.V = zi * U + zr * S.V;
+    double lost;
+    if (!tir) {
+        out.dt = unit((d + n * ci) * M.eta - n * root);
+        const double zt = sqrt((1.0 - Rs) * (1.0 - Rp));
+        out.t.I = S.I - out.r.I;
+        out.t.Q = Q - out.r.Q;
+        out.t.U = zt * U;
+        out.t.V = zt * S.V;
+        lost = rabs(out.r.I + out.t.I - S.I);
+    } else {
+        out.dt = d;
+        out.t = {0.0, 0.0, 0.0, 0.0};
+        lost = rabs(out.r.I - S.I);
+    }
+    out.balance = S.I > 0.0 ? quot(lost, div_by(S.I)) : 0.0;
     return out;
 }
 

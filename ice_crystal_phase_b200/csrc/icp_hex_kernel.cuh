@@ -106,17 +106,46 @@ template <class R> __device__ __forceinline__ R face_offset(const HexGeo<R>& P, 
     return f < 6u ? R(kSqrt3 / 2) : P.half_len;
 }
 
+// Binary64: face normals by selects (the switch above diverges by face).
+template <> __device__ __forceinline__ V3<double> face_normal<double>(unsigned f)
+{
+    const double h = 0.5, s = kSqrt3 / 2;
+    const unsigned k = f >= 3u ? f - 3u : f; // axis of a side face; f < 3 points along it
+    const double x = k == 0u ? 1.0 : (k == 1u ? h : -h), z = k == 0u ? 0.0 : s;
+    const bool side = f < 6u, neg = f >= 3u;
+    return v3(side ? (neg ? -x : x) : 0.0, side ? 0.0 : (f == 6u ? 1.0 : -1.0), side && k ? (neg ? -z : z) : 0.0);
+}
+// Products of v with the prism's four face axes (faces 0, 1, 2 and 6; the opposite faces have the
+// exact negatives).  Equal to the dot products with the normals: a zero component adds nothing.
+struct Axes {
+    double a[4];
+};
+__device__ __forceinline__ Axes prism_axes(V3<double> v)
+{
+    const double h = 0.5, s = kSqrt3 / 2;
+    return {{v.x, h * v.x + s * v.z, -h * v.x + s * v.z, v.y}};
+}
+__device__ __forceinline__ double axis_of(const Axes& A, unsigned f) // product with the normal of face f
+{
+    const unsigned k = f < 6u ? (f >= 3u ? f - 3u : f) : 3u;
+    const double x = k == 0u ? A.a[0] : (k == 1u ? A.a[1] : (k == 2u ? A.a[2] : A.a[3]));
+    return f == 7u || (f >= 3u && f < 6u) ? -x : x;
+}
+
 // hex_prism.hpp:54-57 / 108-120 (FP64 path only): every other face strictly outside tolerance.
 __device__ __forceinline__ bool strict_face_point(const HexGeo<double>& P, V3<double> p, unsigned face)
 {
     const double tol = 128 * Eps<double>::eps * fmax(1.0, fmax(P.half_len, fmax(fabs(p.x), fmax(fabs(p.y), fabs(p.z)))));
-    for (unsigned f = 0; f < 8; ++f) {
-        const double gap = face_offset(P, f) - dot(face_normal<double>(f), p);
-        if (f == face) {
-            if (fabs(gap) > tol) return false;
-        } else if (!(gap > tol)) return false;
+    const Axes A = prism_axes(p);
+    unsigned inside = 1u << face; // faces that p is inside of by more than the tolerance
+#pragma unroll
+    for (unsigned k = 0; k < 4; ++k) {
+        const double off = k < 3 ? kSqrt3 / 2 : P.half_len;
+        inside |= off - A.a[k] > tol ? 1u << (k < 3 ? k : 6u) : 0u;
+        inside |= off + A.a[k] > tol ? 1u << (k < 3 ? k + 3u : 7u) : 0u;
     }
-    return true;
+    const double gap = face_offset(P, face) - axis_of(A, face);
+    return inside == 0xffu && fabs(gap) <= tol;
 }
 
 struct Boundary {
@@ -128,18 +157,12 @@ struct Boundary {
 // Nearest exit plane of the convex prism from a point on `start` (hex_prism.hpp:123-147).
 // FP32: exit t = min over forward-facing planes (no positivity filter, so a point rounded
 // just outside a neighbouring plane exits there at t = 0); near ties are counted only.
-// FP64: the reference rules, ties within geometry tolerance are ambiguous.
+// FP64 (below): the reference rules, ties within geometry tolerance are ambiguous.
 template <class R>
 __device__ __forceinline__ Boundary next_boundary(const HexGeo<R>& P, V3<R>& p, V3<R> d, unsigned start, R& t_out)
 {
     Boundary out{8u, 0, false};
     R best = R(3.0e38), second = R(3.0e38);
-    if constexpr (sizeof(R) == 8) {
-        best = 1.7976931348623157e308;
-        second = best;
-        if (!strict_face_point(P, p, start)) { out.status = 3; return out; }
-        if (dot(face_normal<R>(start), d) > 128 * Eps<double>::eps) { out.status = 5; return out; }
-    }
 #pragma unroll
     for (unsigned f = 0; f < 8; ++f) {
         if (f == start) continue;
@@ -147,24 +170,82 @@ __device__ __forceinline__ Boundary next_boundary(const HexGeo<R>& P, V3<R>& p, 
         const R c = dot(n, d);
         if (!(c > R(0))) continue;
         const R t = (face_offset(P, f) - dot(n, p)) / c;
-        if constexpr (sizeof(R) == 8) {
-            if (!(t > 0) || !finite_r(t)) continue;
-        }
         if (t < best) { second = best; best = t; out.face = f; }
         else if (t < second) second = t;
     }
     if (out.face == 8u) { out.status = 5; return out; }
-    if constexpr (sizeof(R) == 4) {
-        const R t = rmax(best, R(0));
-        p = p + d * t;
-        out.near_edge = (second - best) <= R(64) * Eps<float>::eps * rmax(R(1), P.half_len);
-        t_out = t;
-    } else {
-        p = p + d * best;
-        t_out = best;
-        const double tol = 128 * Eps<double>::eps * fmax(1.0, fmax(P.half_len, fmax(fmax(fabs(p.x), fmax(fabs(p.y), fabs(p.z))), fabs(best))));
-        if (second - best <= tol || !strict_face_point(P, p, out.face)) out.status = 3;
+    const R t = rmax(best, R(0));
+    p = p + d * t;
+    out.near_edge = (second - best) <= R(64) * Eps<float>::eps * rmax(R(1), P.half_len);
+    t_out = t;
+    return out;
+}
+
+// Reciprocal to about 20 bits, for choosing between candidates only.
+__device__ __forceinline__ double rcp_rough(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+
+// FP64.  Of each pair of opposite faces one at most faces forward, so there are four candidates; a
+// rough reciprocal finds the nearest, whose distance is then divided out exactly.  Only when the
+// runner-up is within the rough quotients' error does every candidate get its exact distance (the
+// reference's tie rule needs both).  The point itself was checked against `start` when it
+// was reached (strict_face_point below and at the entry), so it is not checked again here.
+__device__ __forceinline__ Boundary next_boundary(const HexGeo<double>& P, V3<double>& p, V3<double> d, unsigned start,
+                                                  double& t_out)
+{
+    Boundary out{8u, 0, false};
+    const Axes D = prism_axes(d), A = prism_axes(p);
+    if (axis_of(D, start) > 128 * Eps<double>::eps) { out.status = 5; return out; }
+    const double none = 1.7976931348623157e308;
+    double best = none, second = none, gap = 0, slope = 1;
+    double num[4];
+    bool valid[4];
+#pragma unroll
+    for (unsigned k = 0; k < 4; ++k) {
+        const bool fwd = D.a[k] > 0;
+        const unsigned f = k < 3 ? (fwd ? k : k + 3u) : (fwd ? 6u : 7u);
+        const double off = k < 3 ? kSqrt3 / 2 : P.half_len;
+        num[k] = off - (fwd ? A.a[k] : -A.a[k]);
+        valid[k] = D.a[k] != 0 && f != start && num[k] > 0;
+        const double t = valid[k] ? num[k] * rcp_rough(fabs(D.a[k])) : none;
+        const bool less = t < best;
+        second = less ? best : (t < second ? t : second);
+        best = less ? t : best;
+        gap = less ? num[k] : gap;
+        slope = less ? fabs(D.a[k]) : slope;
+        out.face = less ? f : out.face;
     }
+    const double span = fmax(1.0, P.half_len);
+    if (!(second - best > 0x1p-16 * (best + second) + 0x1p-30 * span) || !(best < 0x1p900)) {
+        best = second = none;
+        out.face = 8u;
+#pragma unroll 1
+        for (unsigned f = 0; f < 8; ++f) { // in face order, as the reference
+            const unsigned k = f < 6u ? f % 3u : 3u;
+            const bool fwd = f < 3u || f == 6u;
+            if (f == start) continue;
+            const double ck = k == 0u ? D.a[0] : (k == 1u ? D.a[1] : (k == 2u ? D.a[2] : D.a[3]));
+            const double ak = k == 0u ? A.a[0] : (k == 1u ? A.a[1] : (k == 2u ? A.a[2] : A.a[3]));
+            const double c = fwd ? ck : -ck;
+            if (!(c > 0)) continue;
+            const double t = ((k < 3u ? kSqrt3 / 2 : P.half_len) - (fwd ? ak : -ak)) / c;
+            if (!(t > 0) || !finite_r(t)) continue;
+            if (t < best) { second = best; best = t; out.face = f; }
+            else if (t < second) second = t;
+        }
+        if (out.face == 8u) { out.status = 5; return out; }
+    } else {
+        best = quot(gap, div_by(slope));
+        second = none; // further than the tolerance below
+    }
+    p = p + d * best;
+    t_out = best;
+    const double tol = 128 * Eps<double>::eps * fmax(1.0, fmax(P.half_len, fmax(fmax(fabs(p.x), fmax(fabs(p.y), fabs(p.z))), fabs(best))));
+    if (second - best <= tol || !strict_face_point(P, p, out.face)) out.status = 3;
     return out;
 }
 
@@ -376,6 +457,15 @@ template <class R> __device__ __forceinline__ void lane_acc_clear(LaneAcc<R>& A)
     A.cur_batch_out = 0u;
 }
 
+// Whether idle lanes take their next rays in this step.  The binary64 prism waits for a quarter of
+// the warp (or all of it): its entry is a divergent path of its own, which a step would otherwise run
+// for two or three lanes; the others enter through the code that their live lanes run anyway.
+template <class R, class G> __device__ __forceinline__ bool refill_now(unsigned idle)
+{
+    if constexpr (sizeof(R) == 8 && std::is_same_v<G, HexGeo<R>>) return __popc(idle) >= 8;
+    else return idle != 0u;
+}
+
 // The rays [wnext, wend) of one warp: persistent lanes, one event per lane per step, every
 // exit binned by the whole warp (hex_trace_core.hpp:190-259 per ray).
 template <class R, class G, class P_>
@@ -391,7 +481,7 @@ __device__ __forceinline__ void trace_slice(const P_& P, const BlockShared<R>& B
         // ---- refill idle lanes from the warp's slice
         const unsigned idle = __ballot_sync(kFull, !L.live);
         bool fresh = false;
-        if (idle) {
+        if (refill_now<R, G>(idle)) {
             if (!L.live) {
                 const uint64_t id = wnext + __popc(idle & lt_mask);
                 if (id < wend) { L.id = id; fresh = true; }
