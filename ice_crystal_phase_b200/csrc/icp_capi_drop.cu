@@ -419,6 +419,10 @@ int drop_record(icp_context* c, const icp_drop_record* r, double* phi_out, doubl
                                   (CdfDeviceReport*)c->cdf_report.ptr, (unsigned*)c->cdf_sync.ptr))
         return e;
     ICP_CUDA(cudaEventRecord(c->ev2, c->stream));
+    // the projected area (CPU, binary64) overlaps the device work; the copies below are to pageable
+    // memory and hold the host until the device is done
+    int area_status = ICP_OK;
+    rep->projected_area_mm2 = projected_area_of(r, area_status);
     std::vector<unsigned char> raw(sb);
     CdfDeviceReport cdf{};
     double power = 0;
@@ -436,9 +440,6 @@ int drop_record(icp_context* c, const icp_drop_record* r, double* phi_out, doubl
     } else if (u_out) {
         ICP_CUDA(cudaMemcpyAsync(u_out, coarse.data(), sizeof(double) * (r->ct + 1), cudaMemcpyHostToDevice, c->stream));
     }
-    // the projected area (CPU, binary64) overlaps the device work
-    int area_status = ICP_OK;
-    rep->projected_area_mm2 = projected_area_of(r, area_status);
     ICP_CUDA(cudaStreamSynchronize(c->stream));
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);

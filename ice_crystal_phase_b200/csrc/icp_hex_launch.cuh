@@ -104,20 +104,33 @@ template <class R> TraceParams<R, DropGeo<R>> make_drop_params(const HexLaunch& 
         // half-axes from the extents, scaled by the largest spheroid gauge over 2049 samples of
         // mu, then inflated by 1e-5 (far above the binary32 rounding of the roots and above the
         // sampling error, which is second order in the 9.8e-4 spacing: below 1e-6)
-        const int n = 2048;
+        // the Chebyshev values and sin(chi) of the samples are the same for every shape
+        constexpr int n = 2048;
+        struct Samples {
+            double mu[n + 1], sn[n + 1], t[6][n + 1];
+            Samples()
+            {
+                for (int i = 0; i <= n; ++i) {
+                    mu[i] = -1.0 + 2.0 * i / n;
+                    sn[i] = std::sqrt(std::fmax(0.0, 1 - mu[i] * mu[i]));
+                    double tm = 1, tk = mu[i];
+                    for (int k = 2; k < 8; ++k) {
+                        const double next = 2 * mu[i] * tk - tm;
+                        t[k - 2][i] = next;
+                        tm = tk;
+                        tk = next;
+                    }
+                }
+            }
+        };
+        static const Samples S;
         double ymin = 1e300, ymax = -1e300, hmax = 0;
         std::vector<double> ys(n + 1), hs(n + 1);
         for (int i = 0; i <= n; ++i) {
-            const double mu = -1.0 + 2.0 * i / n;
-            double tm = 1, t = mu, r = 1 + L.coeff[0] + L.coeff[1] * mu;
-            for (int k = 2; k < 8; ++k) {
-                const double tn = 2 * mu * t - tm;
-                r += L.coeff[k] * tn;
-                tm = t;
-                t = tn;
-            }
-            ys[i] = -mu * r;
-            hs[i] = std::sqrt(std::fmax(0.0, 1 - mu * mu)) * r;
+            double r = 1 + L.coeff[0] + L.coeff[1] * S.mu[i];
+            for (int k = 2; k < 8; ++k) r += L.coeff[k] * S.t[k - 2][i];
+            ys[i] = -S.mu[i] * r;
+            hs[i] = S.sn[i] * r;
             ymin = std::fmin(ymin, ys[i]);
             ymax = std::fmax(ymax, ys[i]);
             hmax = std::fmax(hmax, hs[i]);
@@ -126,8 +139,9 @@ template <class R> TraceParams<R, DropGeo<R>> make_drop_params(const HexLaunch& 
         double sc = 0;
         for (int i = 0; i <= n; ++i) {
             const double u = hs[i] / A, v = (ys[i] - y0) / B;
-            sc = std::fmax(sc, std::sqrt(u * u + v * v));
+            sc = std::fmax(sc, u * u + v * v);
         }
+        sc = std::sqrt(sc);
         const double Ae = A * sc * (1 + 1e-5) + 1e-7, Be = B * sc * (1 + 1e-5) + 1e-7;
         P.geo.shape.ea_inv = (R)(1.0 / Ae);
         P.geo.shape.eb_inv = (R)(1.0 / Be);
