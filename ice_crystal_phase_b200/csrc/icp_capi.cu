@@ -510,22 +510,56 @@ int icp::cdf_enqueue(icp_context* c, const double* d_values, uint32_t nt, uint32
     return cdf_launch_common(c, L, ct, cp);
 }
 
+namespace {
+
+// Strips per record of a batched build: 2, or the fewest of 4, 8, .. that fit shared memory (the
+// chains of a strip's columns run side by side, so wider strips cost little and let more records
+// share a launch).  per = records per co-resident launch; 0 when one launch per record is as good.
+// 32 records of 180 x 360 cells stored at 90 x 180: 0.96 ms one by one, 0.06 ms in one launch.
+icp_context::BatchShapeEntry cdf_batch_shape(icp_context* c, uint32_t nt, uint32_t np, uint32_t ct, uint32_t cp)
+{
+    for (const auto& k : c->cdf_batch_shapes)
+        if (k.nt == nt && k.np == np && k.ct == ct && k.cp == cp) return k;
+    icp_context::BatchShapeEntry k{nt, np, ct, cp, 0u, {}};
+    for (uint32_t strips = 2; strips <= 64u && strips <= std::max(2u, cp); strips *= 2u) {
+        if (cdf_choose_shape(c->device, c->sms, nt, np, ct, cp, false, std::max(1u, (cp + strips - 1u) / strips),
+                             0xffffffffu, k.shape))
+            continue;
+        const uint32_t n = (cp + k.shape.cw - 1) / k.shape.cw;
+        k.per = (uint32_t)std::max(0, cdf_max_coresident_blocks(k.shape.smem, c->device)) / n;
+        if (strips > 2u && k.per < 2u) k.per = 0u;
+        break;
+    }
+    c->cdf_batch_shapes.push_back(k);
+    return k;
+}
+
+} // namespace
+
+int icp::cdf_batch_reserve(icp_context* c, uint32_t count, uint32_t nt, uint32_t np, uint32_t ct, uint32_t cp)
+{
+    const auto k = cdf_batch_shape(c, nt, np, ct, cp);
+    if (!k.per) return ICP_OK;
+    const uint32_t strips = (cp + k.shape.cw - 1) / k.shape.cw;
+    ICP_CUDA(c->cdfb_partial.ensure(cdf_partial_bytes() * strips * count));
+    ICP_CUDA(c->cdfb_colsum.ensure(sizeof(double) * cp * count));
+    ICP_CUDA(c->cdfb_recs.ensure(sizeof(CdfBatchRecord) * count));
+    return ICP_OK;
+}
+
 int icp::cdf_enqueue_batch(icp_context* c, const CdfBatchInput* in, uint32_t count, uint32_t nt, uint32_t np,
-                           uint32_t ct, uint32_t cp, const double* d_edges, CdfDeviceReport* d_reports, unsigned* d_sync)
+                           uint32_t ct, uint32_t cp, const double* d_edges, CdfDeviceReport* d_reports, unsigned* d_sync,
+                           CdfBatchRecord* h_staging)
 {
     if (!count) return ICP_OK;
     ICP_CUDA(cudaMemsetAsync(d_sync, 0, 2 * sizeof(unsigned) * count, c->stream));
     ICP_CUDA(cudaMemsetAsync(d_reports, 0, sizeof(CdfDeviceReport) * count, c->stream));
-    // 2 strips per record, as many records per launch as stay co-resident (the chains of a
-    // strip's columns run side by side, so wider strips cost little and let more records share
-    // one launch)
-    CdfShape sh{};
-    const bool fits = cdf_choose_shape(c->device, c->sms, nt, np, ct, cp, false, std::max(1u, (cp + 1u) / 2u),
-                                       0xffffffffu, sh) == 0;
-    const uint32_t strips = fits ? (cp + sh.cw - 1) / sh.cw : 0u;
-    const uint32_t per = fits ? (uint32_t)std::max(0, cdf_max_coresident_blocks(sh.smem, c->device)) / strips : 0u;
+    const auto k = cdf_batch_shape(c, nt, np, ct, cp);
+    const CdfShape& sh = k.shape;
+    const uint32_t per = k.per;
     if (!per) {
-        // a record's strips alone do not fit: one launch per record, with its own strip width
+        // a record's strips alone fill the chip or do not fit: one launch per record, with its own
+        // strip width
         for (uint32_t r = 0; r < count; ++r)
             if (const int e = cdf_enqueue(c, in[r].values, nt, np, ct, cp, d_edges, in[r].fwd_add, in[r].bwd_add,
                                           in[r].pole_fx, in[r].pole_weight, in[r].row_add, in[r].phi, in[r].theta,
@@ -533,11 +567,10 @@ int icp::cdf_enqueue_batch(icp_context* c, const CdfBatchInput* in, uint32_t cou
                 return e;
         return ICP_OK;
     }
-    const size_t pb = cdf_partial_bytes() * strips;
-    ICP_CUDA(c->cdfb_partial.ensure(pb * count));
-    ICP_CUDA(c->cdfb_colsum.ensure(sizeof(double) * cp * count));
-    ICP_CUDA(c->cdfb_recs.ensure(sizeof(CdfBatchRecord) * count));
-    std::vector<CdfBatchRecord> recs(count);
+    if (const int e = cdf_batch_reserve(c, count, nt, np, ct, cp)) return e;
+    const size_t pb = cdf_partial_bytes() * ((cp + sh.cw - 1) / sh.cw);
+    std::vector<CdfBatchRecord> pageable(h_staging ? 0u : count);
+    CdfBatchRecord* recs = h_staging ? h_staging : pageable.data();
     for (uint32_t r = 0; r < count; ++r) {
         CdfBatchRecord& b = recs[r];
         b.values = in[r].values;
@@ -553,7 +586,7 @@ int icp::cdf_enqueue_batch(icp_context* c, const CdfBatchInput* in, uint32_t cou
         b.fwd_add = in[r].fwd_add;
         b.bwd_add = in[r].bwd_add;
     }
-    ICP_CUDA(cudaMemcpyAsync(c->cdfb_recs.ptr, recs.data(), sizeof(CdfBatchRecord) * count, cudaMemcpyHostToDevice,
+    ICP_CUDA(cudaMemcpyAsync(c->cdfb_recs.ptr, recs, sizeof(CdfBatchRecord) * count, cudaMemcpyHostToDevice,
                              c->stream));
     CdfLaunch L{};
     L.edges = d_edges;

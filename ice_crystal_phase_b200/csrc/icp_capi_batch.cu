@@ -2,8 +2,8 @@
 //
 // A batch runs as one device sequence: zero the per-record histograms and counters, one
 // persistent trace launch over all records fed from the chunk queue, the diffraction rows of
-// every record that asks for them (one block per record), and one cooperative CDF build per
-// record reading its pole caps and rows on the device.  With use_graph the sequence is
+// every record that asks for them (one block per record), and the cooperative CDF builds (several
+// records per launch where their strips fit) reading the pole caps and rows on the device.  With use_graph the sequence is
 // captured into a CUDA graph; the executable graph of the previous batch is updated in place
 // when the shape allows (cudaGraphExecUpdate) and re-instantiated otherwise.  The CPU
 // projected-area integrals of all records run on host threads while the device works.
@@ -49,7 +49,13 @@ int ok()
         if (e_ != cudaSuccess) return fail(ICP_ERR_DEVICE, "%s failed: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
-constexpr uint32_t kDefaultChunk = 8192u;
+// Default ray ids per chunk: about eight chunks per resident warp, within 64..1024.  A warp drains
+// its lanes at the end of every chunk, which costs one ray's chain; a batch with fewer chunks than
+// warps leaves the chip idle, which costs more.  32 drops at 180 x 360, chains of 10 (1.6e7 rays):
+// 18.9 ms at 8192, 9.9 at 1024, 9.3 at 256; 1.1e8 rays: 57, 51 and 51 ms; 1.6e5 rays: 16.2, 3.7, 2.2 ms.
+constexpr uint32_t kChunkMin = 64u, kChunkMax = 1024u, kChunksPerWarp = 8u;
+// what icp_drop_batch_autotune starts from
+constexpr uint32_t kTunedChunk = 8192u;
 
 icp_drop_record record_of(const icp_drop_item& it, const icp_batch_settings& s)
 {
@@ -86,20 +92,24 @@ struct Shape {
     uint32_t threads, chunk, blocks;
 };
 
-int launch_shape(icp_context* c, const icp_batch_settings& s, Shape& sh)
+int launch_shape(icp_context* c, const icp_batch_settings& s, uint64_t rays, Shape& sh)
 {
     const BatchState::Tuned* t = tuned_for(c, s.precision, s.nt);
     sh.threads = s.block_threads ? s.block_threads : (t ? t->threads : 256u);
-    sh.chunk = s.chunk_rays ? s.chunk_rays : (t ? t->chunk_rays : kDefaultChunk);
+    sh.chunk = s.chunk_rays ? s.chunk_rays : (t ? t->chunk_rays : 0u);
     if (sh.threads < 64 || sh.threads > 256 || sh.threads % 32)
         return fail(ICP_ERR_INVALID_ARGUMENT, "block_threads must be 64..256, multiple of 32");
-    if (sh.chunk < 32) return fail(ICP_ERR_INVALID_ARGUMENT, "chunk_rays must be at least 32");
-    // a warp flushes its lanes' 32-bit counters once per chunk: keep a chunk within their range
-    sh.chunk = (uint32_t)std::max<uint64_t>(32u, std::min<uint64_t>(sh.chunk, lane_rays_max(s.max_internal_hits)));
+    if (sh.chunk && sh.chunk < 32) return fail(ICP_ERR_INVALID_ARGUMENT, "chunk_rays must be at least 32");
     int per_sm = drop_batch_blocks_per_sm(s.precision, sh.threads, s.nt);
     if (per_sm <= 0) return fail(ICP_ERR_DEVICE, "batch trace kernel cannot be resident");
     if (s.blocks_per_sm) per_sm = std::min<int>(per_sm, (int)s.blocks_per_sm);
     sh.blocks = (uint32_t)per_sm * (uint32_t)c->sms;
+    if (!sh.chunk) {
+        const uint64_t warps = (uint64_t)sh.blocks * (sh.threads / 32u);
+        sh.chunk = (uint32_t)std::min<uint64_t>(kChunkMax, std::max<uint64_t>(kChunkMin, rays / (warps * kChunksPerWarp)));
+    }
+    // a warp flushes its lanes' 32-bit counters once per chunk: keep a chunk within their range
+    sh.chunk = (uint32_t)std::max<uint64_t>(32u, std::min<uint64_t>(sh.chunk, lane_rays_max(s.max_internal_hits)));
     return ICP_OK;
 }
 
@@ -181,7 +191,7 @@ int enqueue_trace(icp_context* c, const icp_drop_item* items, uint32_t count, co
     return ICP_OK;
 }
 
-// Enqueues everything after the trace: diffraction rows, one CDF per record, read-backs.
+// Enqueues everything after the trace: diffraction rows, the CDFs, read-backs.
 int enqueue_finish(icp_context* c, const icp_drop_item* items, uint32_t count, const icp_batch_settings& s,
                    const std::vector<double>& weights, double* d_phi, double* d_theta)
 {
@@ -219,16 +229,22 @@ int enqueue_finish(icp_context* c, const icp_drop_item* items, uint32_t count, c
         count_launch();
         if (e) return fail(ICP_ERR_DEVICE, "diffraction launch failed: %s", cudaGetErrorString((cudaError_t)e));
     }
+    std::vector<CdfBatchInput> in(count);
     for (uint32_t i = 0; i < count; ++i) {
         const unsigned long long* stats = (const unsigned long long*)((unsigned char*)c->b_stats.ptr + sb * i);
-        double* rows = (double*)c->b_rows.ptr + (size_t)(s.nt + 1) * i;
-        if (const int e = cdf_enqueue(c, (const double*)c->b_mass.ptr + cells * i, s.nt, s.np, s.ct, s.cp, d_edges, 0.0,
-                                      0.0, stats + devstats_fwd_word(), weights[i],
-                                      items[i].diffraction ? rows : nullptr, d_phi + (size_t)(s.cp + 1) * i,
-                                      d_theta + (size_t)s.cp * (s.ct + 1) * i,
-                                      (CdfDeviceReport*)c->b_reports.ptr + i, (unsigned*)c->b_sync.ptr + 2 * i))
-            return e;
+        in[i] = CdfBatchInput{(const double*)c->b_mass.ptr + cells * i,
+                              d_phi + (size_t)(s.cp + 1) * i,
+                              d_theta + (size_t)s.cp * (s.ct + 1) * i,
+                              items[i].diffraction ? (double*)c->b_rows.ptr + (size_t)(s.nt + 1) * i : nullptr,
+                              stats + devstats_fwd_word(),
+                              weights[i],
+                              0.0,
+                              0.0};
     }
+    if (const int e = cdf_enqueue_batch(c, in.data(), count, s.nt, s.np, s.ct, s.cp, d_edges,
+                                        (CdfDeviceReport*)c->b_reports.ptr, (unsigned*)c->b_sync.ptr,
+                                        (CdfBatchRecord*)B.h_cdf.ptr))
+        return e;
     ICP_CUDA(cudaMemcpyAsync(B.h_stats.ptr, c->b_stats.ptr, sb * count, cudaMemcpyDeviceToHost, c->stream));
     ICP_CUDA(cudaMemcpyAsync(B.h_reports.ptr, c->b_reports.ptr, sizeof(CdfDeviceReport) * count, cudaMemcpyDeviceToHost,
                              c->stream));
@@ -265,6 +281,8 @@ int prepare(icp_context* c, uint32_t count, const icp_batch_settings& s)
     ICP_CUDA(B.h_stats.ensure(sb * count));
     ICP_CUDA(B.h_reports.ensure(sizeof(CdfDeviceReport) * count));
     ICP_CUDA(B.h_powers.ensure(sizeof(double) * count));
+    ICP_CUDA(B.h_cdf.ensure(sizeof(CdfBatchRecord) * count));
+    if (const int e = cdf_batch_reserve(c, count, s.nt, s.np, s.ct, s.cp)) return e;
     CdfShape sh{};
     const bool tma_ok = s.nt == s.ct && s.np == s.cp && s.np % 2 == 0; // the record histograms are 256-byte aligned
     if (const int e = cdf_shape(c, s.nt, s.np, s.ct, s.cp, tma_ok, sh)) return e;
@@ -327,8 +345,10 @@ int batch(icp_context* c, const icp_drop_item* items, uint32_t count, const icp_
     if (const int v = validate(items, count, settings)) return v;
     const icp_batch_settings& s = *settings;
     ICP_CUDA(cudaSetDevice(c->device));
+    uint64_t rays = 0;
+    for (uint32_t i = 0; i < count; ++i) rays += items[i].rays;
     Shape sh;
-    if (const int e = launch_shape(c, s, sh)) return e;
+    if (const int e = launch_shape(c, s, rays, sh)) return e;
     double* d_phi = phi;
     double* d_theta = theta;
     if (host) {
@@ -453,14 +473,14 @@ extern "C" int icp_drop_batch_autotune(icp_context* c, const icp_drop_item* item
     static const uint32_t kThreads[] = {128u, 256u};
     static const uint32_t kChunks[] = {2048u, 8192u, 32768u};
     double best = 0;
-    uint32_t best_t = 256u, best_c = kDefaultChunk;
+    uint32_t best_t = 256u, best_c = kTunedChunk;
     for (uint32_t t : kThreads)
         for (uint32_t ch : kChunks) {
             icp_batch_settings s = *settings;
             s.block_threads = t;
             s.chunk_rays = ch;
             Shape sh;
-            if (launch_shape(c, s, sh)) continue;
+            if (launch_shape(c, s, rays, sh)) continue;
             if (const int e = prepare(c, n, s)) return e;
             std::vector<double> w;
             double secs = 1e30;

@@ -217,11 +217,15 @@ struct CdfBatchInput {
     double pole_weight, fwd_add, bwd_add;
 };
 // Enqueues the CDF builds of `count` records of one grid shape as few cooperative launches
-// (16 strips per record, as many records per launch as stay co-resident; the records' a / T
-// equal those of one cdf_enqueue per record); d_reports[count] and d_sync[2 count] are zeroed
-// here.  Not for use inside a stream capture (the record table is copied from pageable memory).
+// (the fewest strips per record that fit shared memory, as many records per launch as stay
+// co-resident; the records' a / T equal those of one cdf_enqueue per record); d_reports[count] and
+// d_sync[2 count] are zeroed here.  h_staging: page-locked memory of count CdfBatchRecords that
+// outlives the copy, needed inside a stream capture (null: the record table is copied from
+// pageable memory).  cdf_batch_reserve makes the call's allocations beforehand.
 int cdf_enqueue_batch(icp_context* c, const CdfBatchInput* in, uint32_t count, uint32_t nt, uint32_t np, uint32_t ct,
-                      uint32_t cp, const double* d_edges, CdfDeviceReport* d_reports, unsigned* d_sync);
+                      uint32_t cp, const double* d_edges, CdfDeviceReport* d_reports, unsigned* d_sync,
+                      CdfBatchRecord* h_staging = nullptr);
+int cdf_batch_reserve(icp_context* c, uint32_t count, uint32_t nt, uint32_t np, uint32_t ct, uint32_t cp);
 
 // Analytic diffraction rows of one record on the device (icp_drop_device.cu).
 struct DiffractionArgs {
@@ -277,7 +281,7 @@ struct Pinned {
 };
 // State of the batched-record entries: host staging, the captured graph, tuned launch shapes.
 struct BatchState {
-    Pinned h_table, h_chunks, h_dargs, h_edges, h_stats, h_reports, h_powers;
+    Pinned h_table, h_chunks, h_dargs, h_edges, h_stats, h_reports, h_powers, h_cdf;
     cudaGraphExec_t exec = nullptr;
     struct Tuned {
         uint32_t precision, nt, threads, chunk_rays;
@@ -329,6 +333,12 @@ struct icp_context {
         icp::CdfShape shape;
     };
     std::vector<ShapeEntry> cdf_shapes;
+    // batched builds: (nt, np, ct, cp) -> shape, records per launch (0: one launch per record)
+    struct BatchShapeEntry {
+        uint32_t nt, np, ct, cp, per;
+        icp::CdfShape shape;
+    };
+    std::vector<BatchShapeEntry> cdf_batch_shapes;
     // u edges of the last icp_phase_cdf_enqueue grid (uploaded when nt changes)
     icp::Scratch cdf_edges;
     uint32_t cdf_edges_nt = 0;
