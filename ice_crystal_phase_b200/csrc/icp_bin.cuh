@@ -164,11 +164,13 @@ __device__ __forceinline__ BinResult bin_f32(const BinGridF& g, const float* edg
 }
 
 // ------------------------------------------------------------------ privatised histogram
-// Shared-memory open-addressing table (key = cell + 1, value = fixed-point power), filled by
-// one leader per group of lanes that hit the same cell in a warp step.  Lanes of a group are
-// found with match.any; their 44-bit fixed-point values are summed exactly with two 32-bit
-// redux.sync operations on 22-bit halves.  Inserts that find no slot within kProbe probes go
-// straight to the FP64 global histogram.
+// Shared-memory open-addressing table (key = cell + 1, value = fixed-point power), filled lane by
+// lane.  The 64-bit sums are kept as two 32-bit words with a carry: 32-bit shared additions are
+// native (a 64-bit one is a compare-and-swap loop), and same-cell lanes of a warp cost the hardware
+// its bank conflict only.  Inserts that find no slot within kProbe probes go straight to the FP64
+// global histogram.  (A warp first grouped its lanes by cell with match.any and redux.sync; each
+// group then ran alone, one active lane for most exits: 40 % of the drop kernel's issue slots; the
+// 1e8-ray drop record took 54.9 ms that way and 34.5 ms now.)
 constexpr int kProbe = 8;
 
 struct SmemHist {
@@ -179,41 +181,36 @@ struct SmemHist {
 
 __device__ __forceinline__ uint32_t hash_cell(uint32_t k) { return (k * 0x9E3779B1u) >> 7; }
 
-__device__ __forceinline__ void hist_add(const SmemHist& h, double* global_mass, double to_mass, bool has,
-                                         uint32_t cell, uint64_t v, uint32_t& fallback)
+// sum += v for a 64-bit shared sum that is read after a barrier only.
+__device__ __forceinline__ void add_split(unsigned long long* sum, uint64_t v)
 {
-    const unsigned act = __ballot_sync(kFull, has);
-    if (!act) return;
-    if (has) {
-        const unsigned peers = __match_any_sync(act, cell);
-        const unsigned lo = (unsigned)(v & 0x3FFFFFull), hi = (unsigned)(v >> 22);
-        const unsigned slo = __reduce_add_sync(peers, lo);
-        const unsigned shi = __reduce_add_sync(peers, hi);
-        const unsigned lane = threadIdx.x & 31u;
-        if (lane == (unsigned)(__ffs(peers) - 1)) {
-            const uint64_t sum = ((uint64_t)shi << 22) + (uint64_t)slo;
-            bool done = false;
-            if (h.mask) {
-                const uint32_t key = cell + 1u;
-                uint32_t slot = hash_cell(cell) & h.mask;
+    uint32_t* w = reinterpret_cast<uint32_t*>(sum); // little endian: low word first
+    const uint32_t lo = (uint32_t)v;
+    const uint32_t old = atomicAdd(w, lo);
+    const uint32_t hi = (uint32_t)(v >> 32) + (old + lo < old ? 1u : 0u);
+    if (hi) atomicAdd(w + 1, hi);
+}
+
+// One lane's exit.
+__device__ __forceinline__ void hist_add(const SmemHist& h, double* global_mass, double to_mass, uint32_t cell,
+                                         uint64_t v, uint32_t& fallback)
+{
+    if (h.mask) {
+        const uint32_t key = cell + 1u;
+        uint32_t slot = hash_cell(cell) & h.mask;
 #pragma unroll 1
-                for (int probe = 0; probe < kProbe; ++probe) {
-                    uint32_t k = *((volatile uint32_t*)&h.keys[slot]);
-                    if (k == 0u) k = atomicCAS(&h.keys[slot], 0u, key);
-                    if (k == 0u || k == key) {
-                        atomicAdd(&h.vals[slot], (unsigned long long)sum);
-                        done = true;
-                        break;
-                    }
-                    slot = (slot + 1u) & h.mask;
-                }
+        for (int probe = 0; probe < kProbe; ++probe) {
+            uint32_t k = *((volatile uint32_t*)&h.keys[slot]);
+            if (k == 0u) k = atomicCAS(&h.keys[slot], 0u, key);
+            if (k == 0u || k == key) {
+                add_split(&h.vals[slot], v);
+                return;
             }
-            if (!done) {
-                atomicAdd(&global_mass[cell], (double)sum * to_mass);
-                ++fallback;
-            }
+            slot = (slot + 1u) & h.mask;
         }
     }
+    atomicAdd(&global_mass[cell], (double)v * to_mass);
+    ++fallback;
 }
 
 // Flush the table (after __syncthreads) into the FP64 histogram and clear it.

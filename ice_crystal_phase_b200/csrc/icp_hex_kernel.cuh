@@ -8,9 +8,9 @@
 //   * persistent warps, each owning a contiguous slice of ray ids; a lane whose ray ends
 //     takes the next id of its warp's slice in the next step (no warp idles on long rays);
 //   * one event per lane per step: the entry split, or one internal boundary + split; each
-//     event emits at most one exit, which the whole warp bins together;
-//   * exits go to a shared-memory table through match.any warp aggregation, in 2^-44
-//     fixed point; the table is flushed to FP64 once per block.
+//     event emits at most one exit;
+//   * prism exits go to a shared-memory table in 2^-44 fixed point, flushed to FP64 once per
+//     block; drop exits straight to the FP64 histogram.
 // Ray algorithm: hex_trace/include/ice_crystal/hex_trace_core.hpp:190-259 (linear R/T chain),
 // hex_prism.hpp:64-175 (entry sampling, nearest exit plane), flux_interface.hpp:26-88.
 #pragma once
@@ -467,7 +467,7 @@ template <class R, class G> __device__ __forceinline__ bool refill_now(unsigned 
 }
 
 // The rays [wnext, wend) of one warp: persistent lanes, one event per lane per step, every
-// exit binned by the whole warp (hex_trace_core.hpp:190-259 per ray).
+// exit binned where it is made (hex_trace_core.hpp:190-259 per ray).
 template <class R, class G, class P_>
 __device__ __forceinline__ void trace_slice(const P_& P, const BlockShared<R>& B, uint64_t wnext, const uint64_t wend,
                                             LaneAcc<R>& A)
@@ -637,10 +637,7 @@ __device__ __forceinline__ void trace_slice(const P_& P, const BlockShared<R>& B
             }
         }
 
-        // ---- bin this step's exits (whole warp)
-        uint32_t cell = 0u;
-        bool to_table = false;
-        uint64_t v = 0ull;
+        // ---- bin this step's exits
         if (has) {
             BinResult b;
             if constexpr (sizeof(R) == 4) b = bin_f32(P.gf, B.edges, od);
@@ -648,7 +645,7 @@ __device__ __forceinline__ void trace_slice(const P_& P, const BlockShared<R>& B
             if (!b.valid) {
                 atomicAdd(&T->invalid, 1u);
             } else {
-                v = efx;
+                const uint64_t v = efx;
                 A.esc_fx += v;
                 A.outputs += 1;
                 A.snapped += b.snapped ? 1u : 0u;
@@ -660,12 +657,10 @@ __device__ __forceinline__ void trace_slice(const P_& P, const BlockShared<R>& B
                     if constexpr (power_in_tally<P_>()) atomicAdd(&T->bwd_fx, (unsigned long long)v);
                     else A.bwd_fx += v;
                 } else {
-                    to_table = true;
-                    cell = b.cell;
+                    hist_add(B.H, P.mass, P.to_mass, b.cell, v, A.fallback);
                 }
             }
         }
-        hist_add(B.H, P.mass, P.to_mass, to_table, cell, v, A.fallback);
 
         // ---- per-batch exit counts (the prism's capacity audit), flushed when the lane's batch
         // changes
