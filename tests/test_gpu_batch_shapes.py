@@ -22,12 +22,13 @@ def test_batch_equals_single_records(icp, ctx, nt, np_, ct, cp, count, rays, gra
     specs = icp.batched_record_specs(count, seed=5, rays_max=1e6, rays_min=1e3)
     for sp, n in zip(specs, rays):
         sp.rays = n
-    s = icp.batch_settings(nt, np_, ct, cp, max_internal_hits=10, use_graph=graph)
+    s = icp.batch_settings(nt, np_, ct, cp, max_internal_hits=10, use_graph=graph, precision=icp.ICP_FP64)
     out = icp.generate_drop_batch(ctx, specs, s)
     for i, sp in enumerate(specs):
         one = icp.generate_drop_record(ctx, sp.coefficients, sp.radius_mm, sp.interior_index, nt, np_, sp.rays,
                                        seed=sp.seed, inclination_deg=sp.inclination_deg, ct=ct, cp=cp,
-                                       max_internal_hits=10, wavelength_nm=sp.wavelength_nm, diffraction=sp.diffraction)
+                                       max_internal_hits=10, precision=icp.ICP_FP64, wavelength_nm=sp.wavelength_nm,
+                                       diffraction=sp.diffraction)
         # sums of the same terms in another order: 1e5 rounding errors of 2^-53 at most
         assert np.allclose(out.phi[i], one.phi, rtol=0, atol=1e-11)
         assert np.allclose(out.theta[i], one.theta, rtol=0, atol=1e-11)
