@@ -234,7 +234,7 @@ int drop_trace_enqueue(icp_context* c, const icp_drop_record* r, uint64_t first,
 {
     const bool f32 = r->precision == ICP_FP32;
     const uint32_t max_threads = f32 ? drop_trace_threads_f32() : drop_trace_threads_f64();
-    const uint32_t threads = r->tuning.block_threads ? r->tuning.block_threads : max_threads;
+    const uint32_t threads = r->tuning.block_threads ? r->tuning.block_threads : 128u; // see TraceShape
     if (threads < 64 || threads > max_threads || threads % 32)
         return fail(ICP_ERR_INVALID_ARGUMENT, "block_threads must be 64..%u, multiple of 32", max_threads);
     uint32_t slots;

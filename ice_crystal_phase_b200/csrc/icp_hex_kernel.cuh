@@ -748,12 +748,16 @@ __device__ __forceinline__ void block_flush(const P_& P, const BlockShared<R>& B
 
 // Block shape of the single-record trace: the FP32 drop runs 128-thread blocks, seven per SM at
 // 72 registers (fewer spills than four 256-thread blocks at 64 registers: 1 % faster); the FP32
-// prism keeps four 256-thread blocks (its 48 KB shared histogram table per block), the FP64
-// kernels 256 threads.
+// prism keeps four 256-thread blocks (its 48 KB shared histogram table per block).  The FP64 kernels
+// wait on chains of dependent operations: the prism runs two 256-thread blocks at 128 registers (1e6
+// rays over two orientations 3.87 ms with one block at 162, 3.04 with two, 3.44 with three at 80 and
+// their spills), the drop three 128-thread blocks at 162 registers (fewer registers lengthen the
+// long chains that small records wait for).
 template <class R, class G> struct TraceShape {
-    static constexpr bool drop32 = sizeof(R) == 4 && !std::is_same_v<G, HexGeo<R>>;
-    static constexpr unsigned threads = drop32 ? 128u : 256u;
-    static constexpr unsigned min_blocks = sizeof(R) == 4 ? (drop32 ? 7u : 4u) : 1u;
+    static constexpr bool hex = std::is_same_v<G, HexGeo<R>>;
+    static constexpr bool drop32 = sizeof(R) == 4 && !hex;
+    static constexpr unsigned threads = drop32 ? 128u : 256u; // the largest block
+    static constexpr unsigned min_blocks = sizeof(R) == 4 ? (drop32 ? 7u : 4u) : (hex ? 2u : 1u);
 };
 
 // One record: the ray range [first, first+count) split into contiguous per-warp slices.

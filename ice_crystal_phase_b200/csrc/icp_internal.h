@@ -325,6 +325,11 @@ struct icp_context {
     // atlas composition: the compacted nonzero coupling shifts
     icp::Scratch atlas_list;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
+    // further streams of one call whose launches are independent (the orientation nodes of a prism
+    // record); every call that uses them joins them into `stream` before it returns
+    static constexpr int kSide = 3;
+    cudaStream_t side[kSide] = {};
+    cudaEvent_t fork = nullptr, join[kSide] = {};
     // grid-barrier iteration limit handed to the CDF kernels (0: their default)
     uint32_t wait_limit = 0;
     // CDF launch shapes already chosen: (nt, np, ct, cp, tma allowed) -> shape
