@@ -17,9 +17,9 @@
 //   atlas_compose_kernel   out[t][p] = sum_(n,q,s) w[n][q][s] * M_n[t][(p - s) mod np]
 //                          (phi reflected when q = 1) over the nonzero shifts only, compacted
 //                          per (node, parity) in shift order by atlas_weights_compact_kernel
-//                          (the couplings are ~4 % nonzero); kTT rows of a node in shared
-//                          memory, a thread per cell column; products and sums are rounded
-//                          separately in the order node, parity, shift -- the order of
+//                          (the couplings are ~4 % nonzero), two neighbouring shifts to an
+//                          entry; a block per row, the row in shared memory, a thread per K
+//                          consecutive cells; products and sums are rounded separately in the order node, parity, shift -- the order of
 //                          compose_mass's elementwise `out += value * roll(cell)`
 //                          (atlas_math.py:431-447), so equal weights give equal bits.
 #include <algorithm>
@@ -319,137 +319,160 @@ __global__ void __launch_bounds__(128) atlas_coupling_kernel(const AtlasCoupling
     atomicAdd(P.expected, __double2ull_rn(base * P.inv_unit));
 }
 
-// One warp per [node][parity] row: fixed point -> weights per node area; optional exact
-// orbit average (the row's mean, summed in a fixed order); out += fraction * row.
-__global__ void __launch_bounds__(256) atlas_coupling_finish_kernel(const unsigned long long* acc,
-                                                                    const double* node_area, uint32_t rows,
-                                                                    uint32_t np, double unit, double fraction,
-                                                                    int orbit, double* out)
+// One block per [node][parity] row: fixed point -> weights per node area; optional exact orbit average
+// (the row's mean, summed by one warp in a fixed order); out += fraction * row.  (One warp per row
+// left seven blocks on the chip: 37 us for 56 rows of 1800.)
+constexpr int kFinishThreads = 256;
+__global__ void __launch_bounds__(kFinishThreads) atlas_coupling_finish_kernel(const unsigned long long* acc,
+                                                                               const double* node_area, uint32_t np,
+                                                                               double unit, double fraction, int orbit,
+                                                                               double* out)
 {
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    if (warp >= rows) return;
-    const double scale = unit / node_area[warp >> 1];
-    const unsigned long long* a = acc + (uint64_t)warp * np;
-    double* o = out + (uint64_t)warp * np;
+    const uint32_t row = blockIdx.x;
+    const double scale = unit / node_area[row >> 1];
+    const unsigned long long* a = acc + (uint64_t)row * np;
+    double* o = out + (uint64_t)row * np;
     if (orbit) {
-        double part = 0;
-        for (uint32_t s = lane; s < np; s += 32) part += (double)a[s] * scale;
-        for (int d = 16; d; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
-        const double mean = part / np;
-        for (uint32_t s = lane; s < np; s += 32) o[s] += fraction * mean;
+        __shared__ double mean;
+        if (threadIdx.x < 32) {
+            double part = 0;
+            for (uint32_t s = threadIdx.x; s < np; s += 32) part += (double)a[s] * scale;
+            for (int d = 16; d; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
+            if (threadIdx.x == 0) mean = part / np;
+        }
+        __syncthreads();
+        for (uint32_t s = threadIdx.x; s < np; s += kFinishThreads) o[s] += fraction * mean;
     } else {
-        for (uint32_t s = lane; s < np; s += 32) o[s] += fraction * ((double)a[s] * scale);
+        for (uint32_t s = threadIdx.x; s < np; s += kFinishThreads) o[s] += fraction * ((double)a[s] * scale);
     }
 }
 
 // ------------------------------------------------------------------ compose
-constexpr int kTT = 2;                 // rows per block
-constexpr int kComposeThreads = 256;   // cells per block row: threads x CPT >= np
 constexpr int kCompactThreads = 256;
+constexpr uint32_t kMaxPhi = 4096; // cells per row
 
-// The nonzero shifts of one (node, parity) coupling row, ascending, with their weights: one
-// block per row, ballot ranks within each warp and the warps' counts in order, so the list's
-// order is the shift order (the composition's summation order depends on it).
+// The nonzero shifts of one (node, parity) coupling row in ascending order, two neighbouring shifts
+// to an entry: (shift s, weights of s and s + 1), the second zero where s + 1 has none.  A fractional
+// shift puts its weight on two neighbours, so nearly all entries are full.  One block per row.
 __global__ void __launch_bounds__(kCompactThreads) atlas_weights_compact_kernel(const double* __restrict__ w, uint32_t np,
                                                                                 uint32_t* __restrict__ counts,
                                                                                 uint32_t* __restrict__ shifts,
-                                                                                double* __restrict__ values)
+                                                                                double2* __restrict__ values)
 {
-    __shared__ uint32_t warp_count[kCompactThreads / 32];
-    __shared__ uint32_t base;
-    const uint32_t row = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    __shared__ uint32_t nonzero[kMaxPhi / 32], heads[kMaxPhi / 32], before[kMaxPhi / 32 + 1];
+    const uint32_t row = blockIdx.x, lane = threadIdx.x & 31u, words = (np + 31u) / 32u;
     const double* wr = w + (uint64_t)row * np;
-    if (threadIdx.x == 0) base = 0;
-    __syncthreads();
-    for (uint32_t s0 = 0; s0 < np; s0 += kCompactThreads) {
-        const uint32_t sft = s0 + threadIdx.x;
-        const double v = sft < np ? wr[sft] : 0.0;
-        const bool nz = v != 0.0;
-        const unsigned ballot = __ballot_sync(0xffffffffu, nz);
-        if (lane == 0) warp_count[warp] = __popc(ballot);
-        __syncthreads();
-        uint32_t before = base;
-        for (uint32_t k = 0; k < warp; ++k) before += warp_count[k];
-        if (nz) {
-            const uint32_t slot = before + __popc(ballot & ((1u << lane) - 1u));
-            shifts[(uint64_t)row * np + slot] = sft;
-            values[(uint64_t)row * np + slot] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0)
-            for (uint32_t k = 0; k < kCompactThreads / 32; ++k) base += warp_count[k];
-        __syncthreads();
+    for (uint32_t k = threadIdx.x >> 5; k < words; k += kCompactThreads / 32) {
+        const uint32_t s = k * 32u + lane;
+        const unsigned bits = __ballot_sync(0xffffffffu, s < np && wr[s] != 0.0);
+        if (lane == 0) nonzero[k] = bits;
     }
-    if (threadIdx.x == 0) counts[row] = base;
+    __syncthreads();
+    // the shifts at an even offset of their run start an entry
+    for (uint32_t k = threadIdx.x >> 5; k < words; k += kCompactThreads / 32) {
+        uint32_t z = ~nonzero[k] & ((1u << lane) - 1u); // zeros below this shift
+        uint32_t j = k;
+        while (!z && j > 0) z = ~nonzero[--j];
+        const uint32_t start = z ? j * 32u + 32u - (uint32_t)__clz((int)z) : 0u; // first shift of the run
+        const bool head = ((nonzero[k] >> lane) & 1u) && (k * 32u + lane - start) % 2u == 0u;
+        const unsigned bits = __ballot_sync(0xffffffffu, head);
+        if (lane == 0) heads[k] = bits;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t n = 0;
+        for (uint32_t k = 0; k < words; ++k) {
+            before[k] = n;
+            n += __popc(heads[k]);
+        }
+        counts[row] = n;
+    }
+    __syncthreads();
+    for (uint32_t s = threadIdx.x; s < np; s += kCompactThreads) {
+        const uint32_t k = s >> 5, bit = s & 31u;
+        if (!((heads[k] >> bit) & 1u)) continue;
+        const uint64_t slot = (uint64_t)row * np + before[k] + __popc(heads[k] & ((1u << bit) - 1u));
+        shifts[slot] = s;
+        values[slot] = make_double2(wr[s], s + 1u < np ? wr[s + 1u] : 0.0);
+    }
+}
+
+// Shared memory of the composition: one row twice over and the reach of the last thread.
+__host__ __device__ constexpr uint32_t compose_cells(uint32_t np, uint32_t threads, uint32_t k)
+{
+    return np + threads * k + 1u;
 }
 
 // out[t][p] = sum over nodes n, parities q and the nonzero shifts s of w[n][q][s] *
-// M_n[t][(p - s) mod np] (phi-reflected when q = 1).  A block holds kTT rows of one node in
-// shared memory and the (n, q) list of nonzero shifts; thread x owns the cells x + k T of its
-// rows (consecutive threads read consecutive cells).  Products and sums rounded separately,
-// in the order node, parity, ascending shift -- the order of compose_mass's elementwise
+// M_n[t][(p - s) mod np] (phi-reflected when q = 1).  Products and sums rounded separately, in the
+// order node, parity, ascending shift -- the order of compose_mass's elementwise
 // `out += value * roll(cell)` (atlas_math.py:431-447), so equal weights give equal bits.
-template <int CPT>
-__global__ void __launch_bounds__(kComposeThreads, 2) atlas_compose_kernel(const double* __restrict__ mass,
-                                                                           const uint32_t* __restrict__ counts,
-                                                                           const uint32_t* __restrict__ shifts,
-                                                                           const double* __restrict__ values,
-                                                                           uint32_t nodes, uint32_t nt, uint32_t np,
-                                                                           double* __restrict__ out)
+//
+// A block composes one row; thread x owns the K consecutive cells from K x on.  The row (reflected for
+// q = 1) lies in shared memory with its head repeated behind its tail, so a cell is a plain offset and
+// no index wraps.  The K + 1 cells of an entry serve its two shifts, 2 K products: shared memory
+// delivers half a warp's cells per cycle and the FP64 pipe consumes one product and sum, so a load per
+// product would bound the kernel at twice its FP64 time; K is odd, which keeps the stride of the
+// threads' loads free of bank conflicts.  28 nodes at 900 x 1800, 3900 weights (0.7 ms of FP64 issue, 0.8
+// of shared-memory loads): 3.09 ms with a load and index arithmetic per product, 1.45 ms now.
+constexpr uint32_t kStage = 128; // entries in shared memory at a time
+template <int K>
+__global__ void __launch_bounds__(256) atlas_compose_kernel(const double* __restrict__ mass,
+                                                            const uint32_t* __restrict__ counts,
+                                                            const uint32_t* __restrict__ shifts,
+                                                            const double2* __restrict__ values, uint32_t nodes,
+                                                            uint32_t nt, uint32_t np, double* __restrict__ out)
 {
-    extern __shared__ __align__(16) double sm[];
-    double* rows = sm;                                             // [kTT][np]
-    double* lw = sm + kTT * np;                                    // [np] weights of the list
-    uint32_t* ls = reinterpret_cast<uint32_t*>(lw + np);           // [np] shifts of the list
-    const uint32_t t0 = blockIdx.x * kTT;
-    double acc[kTT][CPT];
+    extern __shared__ __align__(16) double row[]; // [compose_cells]: row[np + m] = row[m] = cell m
+    __shared__ double2 s_w[kStage];               // entries: weights, np - 1 - shift
+    __shared__ uint32_t s_from[kStage];
+    const uint32_t t = blockIdx.x, x0 = threadIdx.x * K, cells = compose_cells(np, blockDim.x, K);
+    double acc[K];
 #pragma unroll
-    for (int t = 0; t < kTT; ++t)
-#pragma unroll
-        for (int k = 0; k < CPT; ++k) acc[t][k] = 0.0;
+    for (int k = 0; k < K; ++k) acc[k] = 0.0;
     for (uint32_t n = 0; n < nodes; ++n) {
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < kTT * np; e += blockDim.x) {
-            const uint32_t t = t0 + e / np;
-            rows[e] = t < nt ? mass[((uint64_t)n * nt + t) * np + e % np] : 0.0;
-        }
+        const double* src = mass + ((uint64_t)n * nt + t) * np;
         for (int q = 0; q < 2; ++q) {
             const uint64_t r = (uint64_t)n * 2 + q;
             const uint32_t cnt = counts[r];
-            __syncthreads();
-            for (uint32_t e = threadIdx.x; e < cnt; e += blockDim.x) {
-                lw[e] = values[r * np + e];
-                ls[e] = shifts[r * np + e];
-            }
-            __syncthreads();
-            if (threadIdx.x < np)
-                for (uint32_t e = 0; e < cnt; ++e) {
-                    const double wv = lw[e];
-                    // m = (p - s) mod np for p = x + k T, stepped by T per cell (T < np when CPT > 1)
-                    uint32_t m = phi_sub(threadIdx.x, ls[e], np);
+            if (!cnt) continue;
+            const uint32_t* ls = shifts + r * np;
+            const double2* lw = values + r * np;
+            for (uint32_t e0 = 0; e0 < cnt; e0 += kStage) {
+                __syncthreads(); // the previous row and entries are no longer read
+                if (e0 == 0)
+                    for (uint32_t e = threadIdx.x; e < np; e += blockDim.x) {
+                        const double v = src[e];
+                        for (uint32_t c = phi_cell(e, np, q); c < cells; c += np) row[c] = v;
+                    }
+                const uint32_t batch = min(kStage, cnt - e0);
+                for (uint32_t e = threadIdx.x; e < batch; e += blockDim.x) {
+                    s_w[e] = lw[e0 + e];
+                    s_from[e] = np - 1u - ls[e0 + e];
+                }
+                __syncthreads();
+                for (uint32_t e = 0; e < batch; ++e) {
+                    const double2 w = s_w[e];
+                    const double* from = row + (s_from[e] + x0); // cell x0 - s - 1
+                    double v[K + 1];
 #pragma unroll
-                    for (int k = 0; k < CPT; ++k) {
-                        if (k > 0) {
-                            if (threadIdx.x + (uint32_t)k * kComposeThreads >= np) break;
-                            m += kComposeThreads;
-                            if (m >= np) m -= np;
-                        }
-                        const uint32_t idx = phi_cell(m, np, q);
+                    for (int k = 0; k <= K; ++k) v[k] = from[k];
 #pragma unroll
-                        for (int t = 0; t < kTT; ++t) acc[t][k] = acc[t][k] + wv * rows[t * np + idx];
+                    for (int k = 0; k < K; ++k) acc[k] = acc[k] + w.x * v[k + 1];
+                    if (w.y != 0.0) {
+#pragma unroll
+                        for (int k = 0; k < K; ++k) acc[k] = acc[k] + w.y * v[k];
                     }
                 }
+            }
         }
     }
+    // contiguous stores through shared memory
+    __syncthreads();
 #pragma unroll
-    for (int t = 0; t < kTT; ++t) {
-        if (t0 + t >= nt) continue;
-#pragma unroll
-        for (int k = 0; k < CPT; ++k) {
-            const uint32_t p = threadIdx.x + (uint32_t)k * kComposeThreads;
-            if (p < np) out[(uint64_t)(t0 + t) * np + p] = acc[t][k];
-        }
-    }
+    for (int k = 0; k < K; ++k) row[x0 + k] = acc[k];
+    __syncthreads();
+    for (uint32_t p = threadIdx.x; p < np; p += blockDim.x) out[(uint64_t)t * np + p] = row[p];
 }
 
 int validate_settings(const icp_atlas_settings* s)
@@ -707,9 +730,8 @@ int icp_atlas_coupling(icp_context* ctx, uint32_t it, uint32_t ip, uint32_t np, 
     ICP_CUDA(cudaGetLastError());
     count_launch();
     const uint32_t rows = (uint32_t)(nodes * 2);
-    atlas_coupling_finish_kernel<<<(rows * 32 + 255) / 256, 256, 0, stream>>>(d_acc, d_area, rows, np,
-                                                                             bound * kUnit62, fraction,
-                                                                             orbit_average, d_coupling);
+    atlas_coupling_finish_kernel<<<rows, kFinishThreads, 0, stream>>>(d_acc, d_area, np, bound * kUnit62, fraction,
+                                                                     orbit_average, d_coupling);
     ICP_CUDA(cudaGetLastError());
     count_launch();
     unsigned long long tail[4];
@@ -730,37 +752,36 @@ int icp_atlas_compose(icp_context* ctx, uint32_t nodes, uint32_t nt, uint32_t np
     if (!ctx || !d_mass || !d_coupling || !d_out) return fail(ICP_ERR_INVALID_ARGUMENT, "icp_atlas_compose: null argument");
     if (nodes == 0 || nt == 0 || np == 0 || uint64_t(nt) * np > 100000000ull)
         return fail(ICP_ERR_INVALID_ARGUMENT, "icp_atlas_compose: invalid shape");
-    const size_t smem = (size_t(kTT) + 1) * np * sizeof(double) + np * sizeof(uint32_t);
-    if (smem > 227u * 1024u || np > 16u * kComposeThreads)
-        return fail(ICP_ERR_CAPACITY, "icp_atlas_compose: %u phi cells need %zu bytes of shared memory (limit 227 KiB) "
-                    "or more than %u cells per row", np, smem, 16u * kComposeThreads);
+    if (np > kMaxPhi)
+        return fail(ICP_ERR_CAPACITY, "icp_atlas_compose: %u phi cells (at most %u per row)", np, kMaxPhi);
     ICP_CUDA(cudaSetDevice(ctx->device));
     // the nonzero coupling shifts of every (node, parity) row, compacted in shift order
     const uint64_t rowsw = uint64_t(nodes) * 2;
     const size_t o_shifts = (rowsw * 4 + 255) / 256 * 256, o_values = o_shifts + (rowsw * np * 4 + 255) / 256 * 256;
-    ICP_CUDA(ctx->atlas_list.ensure(o_values + rowsw * np * 8));
+    ICP_CUDA(ctx->atlas_list.ensure(o_values + rowsw * np * sizeof(double2)));
     char* base = static_cast<char*>(ctx->atlas_list.ptr);
     auto* counts = reinterpret_cast<uint32_t*>(base);
     auto* shifts = reinterpret_cast<uint32_t*>(base + o_shifts);
-    auto* values = reinterpret_cast<double*>(base + o_values);
+    auto* values = reinterpret_cast<double2*>(base + o_values);
     atlas_weights_compact_kernel<<<(unsigned)rowsw, kCompactThreads, 0, ctx->stream>>>(d_coupling, np, counts, shifts,
                                                                                       values);
     ICP_CUDA(cudaGetLastError());
     count_launch();
-    const uint32_t cpt = (np + kComposeThreads - 1) / kComposeThreads;
-    const dim3 grid((nt + kTT - 1) / kTT);
-    auto run = [&](auto kernel) -> cudaError_t {
+    auto run = [&](auto kernel, uint32_t k) -> cudaError_t {
+        const uint32_t threads = (((np + k - 1) / k) + 31u) / 32u * 32u;
+        const size_t smem = compose_cells(np, threads, k) * sizeof(double);
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kernel<<<grid, kComposeThreads, smem, ctx->stream>>>(d_mass, counts, shifts, values, nodes, nt, np, d_out);
+        kernel<<<nt, threads, smem, ctx->stream>>>(d_mass, counts, shifts, values, nodes, nt, np, d_out);
         return cudaGetLastError();
     };
+    // K = 9 keeps the most warps per row that the loads still serve twice (28 nodes at 900 x 1800: 1.60 ms
+    // a record, 1.76 with K = 15, 1.93 with K = 19); rows beyond 256 threads of 9 need 17, and fewer
+    // rows than two per SM take 5 for the warps
     cudaError_t e;
-    if (cpt <= 1) e = run(atlas_compose_kernel<1>);
-    else if (cpt <= 2) e = run(atlas_compose_kernel<2>);
-    else if (cpt <= 4) e = run(atlas_compose_kernel<4>);
-    else if (cpt <= 8) e = run(atlas_compose_kernel<8>);
-    else e = run(atlas_compose_kernel<16>);
+    if (np > 9u * 256u) e = run(atlas_compose_kernel<17>, 17u);
+    else if (nt < 2u * (uint32_t)ctx->sms && np <= 5u * 256u) e = run(atlas_compose_kernel<5>, 5u);
+    else e = run(atlas_compose_kernel<9>, 9u);
     ICP_CUDA(e);
     count_launch();
     ICP_CUDA(cudaStreamSynchronize(ctx->stream));
