@@ -4,15 +4,16 @@
 // of one training step, a prediction and a generated record.
 //
 // Training step over R records (M = R * nt * np rows, H hidden units, K0 input width):
-//   X, XT                          feature rows (row- and column-major)
-//   L1  X  W1^T  (kHidden)         z1, h1, h1T
-//   L2  h1 W2^T  (kHidden)         z2, h2, h2T
+//   X                              feature rows
+//   L1  X  W1^T  (kHidden)         z1, h1
+//   L2  h1 W2^T  (kHidden)         z2, h2
 //   L3  h2 W3^T  (kHead)           z3, y = silu(z3) . w4 + head bias
 //   softmax per record             dy = (softmax(y) - p) / R, KL loss
-//   head backward                  dz3, dz3T, dw4, db3
-//   dW3 = dz3T h2T^T (split-K)     dz2 = (dz3 W3) silu'(z2)  -> dz2, dz2T, db2     (kBackprop)
-//   dW2 = dz2T h1T^T (split-K)     dz1 = (dz2 W2) silu'(z1)  -> dz1T, db1           (kBackprop)
-//   dW1 = dz1T XT^T  (split-K)     Adam, BF16 copies of W1, W2, W3, W2^T, W3^T
+//   head backward                  dz3, dw4, db3
+//   dW3 = dz3^T h2 (weight_grad)   dz2 = (dz3 W3) silu'(z2)  -> dz2, db2     (kBackprop)
+//   dW2 = dz2^T h1                 dz1 = (dz2 W2) silu'(z1)  -> dz1, db1     (kBackprop)
+//   dW1 = dz1^T X                  Adam, BF16 copies of W1, W2, W3, W2^T, W3^T
+// Every matrix is row-major; the weight gradients contract over the rows (MN-major operands).
 // A generated record: L1, L2, L3 with the head writing exp(y) as the FP64 cell mass, then the
 // cooperative CDF build of each record.
 #include <algorithm>
@@ -156,7 +157,7 @@ struct icp_surrogate {
     float head_b = 0.0f;
     uint32_t o_w1 = 0, o_b1 = 0, o_w2 = 0, o_b2 = 0, o_w3 = 0, o_b3 = 0, o_w4 = 0, o_hb = 0;
     Scratch params, grads, adam_m, adam_v, wbf, cells, edges, rec16, loss;
-    Scratch X, XT, z1, h1, h1T, z2, h2, h2T, z3, y, dy, dz3, dz3T, dz2, dz2T, dz1T, mass, reports, sync;
+    Scratch X, z1, h1, z2, h2, z3, y, dy, dz3, dz2, dz1, mass, reports, sync;
     Scratch mass_sum, dfrac, drows, cellgeo, recgeo, xcells;
     std::vector<double> h_edges;
     std::vector<uint16_t> h_rec;
@@ -166,8 +167,8 @@ struct icp_surrogate {
     {
         h_frac.release();
         h_reports.release();
-        Scratch* all[] = {&params, &grads, &adam_m, &adam_v, &wbf, &cells, &edges, &rec16, &loss, &X, &XT, &z1, &h1,
-                          &h1T, &z2, &h2, &h2T, &z3, &y, &dy, &dz3, &dz3T, &dz2, &dz2T, &dz1T, &mass, &reports, &sync,
+        Scratch* all[] = {&params, &grads, &adam_m, &adam_v, &wbf, &cells, &edges, &rec16, &loss, &X, &z1, &h1,
+                          &z2, &h2, &z3, &y, &dy, &dz3, &dz2, &dz1, &mass, &reports, &sync,
                           &mass_sum, &dfrac, &drows, &cellgeo, &recgeo, &xcells};
         for (Scratch* s : all) s->release();
     }
@@ -196,9 +197,9 @@ int check_call(icp_surrogate* s, const icp_drop_item* items, uint32_t count)
 // Inference runs as one fused kernel that builds its own input rows (mlp::forward_fused).
 bool fused_inference(const icp_surrogate* s) { return mlp::fused_shape(s->K0, s->H); }
 
-// Record feature rows to the device and the feature matrix (XT too when training; no matrix
-// when `rows` is false: the fused inference pass builds the rows itself).
-int enqueue_features(icp_surrogate* s, const icp_drop_item* items, uint32_t count, bool training, bool rows = true)
+// Record feature rows to the device and the feature matrix (no matrix when `rows` is false: the
+// fused inference pass builds the rows itself).
+int enqueue_features(icp_surrogate* s, const icp_drop_item* items, uint32_t count, bool rows = true)
 {
     icp_context* c = s->c;
     s->h_rec.resize((size_t)16 * count);
@@ -216,13 +217,10 @@ int enqueue_features(icp_surrogate* s, const icp_drop_item* items, uint32_t coun
     ICP_CUDA(cudaMemcpyAsync(s->recgeo.ptr, s->h_recgeo.data(), 16u * count, cudaMemcpyHostToDevice, c->stream));
     if (!rows) return ICP_OK;
     ICP_CUDA(s->X.ensure(2 * M * s->K0));
-    if (training) ICP_CUDA(s->XT.ensure(2 * M * s->K0));
     const int e = mlp::launch_features(as<__nv_bfloat16>(s->rec16), as<__nv_bfloat16>(s->cells), count, s->C, s->K0,
                                        s->cfg.axis_harmonics, as<double>(s->recgeo), as<double>(s->cellgeo),
-                                       as<__nv_bfloat16>(s->X), training ? as<__nv_bfloat16>(s->XT) : nullptr,
-                                       c->stream);
+                                       as<__nv_bfloat16>(s->X), c->stream);
     count_launch();
-    if (training) count_launch();
     if (e) return fail(ICP_ERR_DEVICE, "feature launch failed (%d)", e);
     return ICP_OK;
 }
@@ -236,17 +234,25 @@ int run_gemm(icp_surrogate* s, const void* A, const void* B, mlp::GemmArgs g, in
     return ICP_OK;
 }
 
+int run_weight_grad(icp_surrogate* s, const void* A, const void* B, mlp::GemmArgs g, uint32_t splits)
+{
+    g.error = (unsigned*)s->c->mlp_error.ptr;
+    const int e = mlp::weight_grad(A, B, g, splits, s->c->stream);
+    count_launch();
+    if (e) return fail(ICP_ERR_DEVICE, "surrogate weight-gradient launch failed (%d)", e);
+    return ICP_OK;
+}
+
 mlp::GemmArgs layer(uint64_t M, uint32_t N, uint32_t K)
 {
     mlp::GemmArgs g{};
     g.M = (uint32_t)M;
     g.N = N;
     g.K = K;
-    g.ld_t = (uint32_t)M;
     return g;
 }
 
-// Forward pass.  training: keep z1, z2, z3 and the column-major activations; else the head
+// Forward pass.  training: keep z1, z2, z3, h1, h2; else the head
 // writes y (logits) or exp(y) (mass).
 int enqueue_forward(icp_surrogate* s, uint32_t count, bool training, float* y_out, double* mass_out,
                     double* mass_sum = nullptr)
@@ -282,25 +288,19 @@ int enqueue_forward(icp_surrogate* s, uint32_t count, bool training, float* y_ou
     ICP_CUDA(s->h1.ensure(act));
     ICP_CUDA(s->h2.ensure(act));
     if (training) {
-        Scratch* t[] = {&s->z1, &s->h1T, &s->z2, &s->h2T, &s->z3};
+        Scratch* t[] = {&s->z1, &s->z2, &s->z3};
         for (Scratch* x : t) ICP_CUDA(x->ensure(act));
     }
     mlp::GemmArgs g = layer(M, Hn, s->K0);
     g.bias = s->P(s->o_b1);
     g.out_h = as<__nv_bfloat16>(s->h1);
-    if (training) {
-        g.out_z = as<__nv_bfloat16>(s->z1);
-        g.out_hT = as<__nv_bfloat16>(s->h1T);
-    }
+    if (training) g.out_z = as<__nv_bfloat16>(s->z1);
     const int hid = training ? mlp::kHiddenTrain : mlp::kHidden;
     ICP_TRY(run_gemm(s, s->X.ptr, s->w1b(), g, hid, 1));
     g = layer(M, Hn, Hn);
     g.bias = s->P(s->o_b2);
     g.out_h = as<__nv_bfloat16>(s->h2);
-    if (training) {
-        g.out_z = as<__nv_bfloat16>(s->z2);
-        g.out_hT = as<__nv_bfloat16>(s->h2T);
-    }
+    if (training) g.out_z = as<__nv_bfloat16>(s->z2);
     ICP_TRY(run_gemm(s, s->h1.ptr, s->w2b(), g, hid, 1));
     g = layer(M, Hn, Hn);
     g.bias = s->P(s->o_b3);
@@ -331,45 +331,44 @@ int enqueue_backward(icp_surrogate* s, uint32_t count)
     const uint64_t M = (uint64_t)count * s->C;
     const uint32_t Hn = s->H;
     const size_t act = 2 * M * Hn;
-    Scratch* t[] = {&s->dz3, &s->dz3T, &s->dz2, &s->dz2T, &s->dz1T};
+    Scratch* t[] = {&s->dz3, &s->dz2, &s->dz1};
     for (Scratch* x : t) ICP_CUDA(x->ensure(act));
     ICP_CUDA(cudaMemsetAsync(s->grads.ptr, 0, 4 * s->n_params, c->stream));
     int e = mlp::launch_head_backward(as<__nv_bfloat16>(s->z3), as<float>(s->dy), s->P(s->o_w4), (uint32_t)M, Hn,
-                                      as<__nv_bfloat16>(s->dz3), as<__nv_bfloat16>(s->dz3T), s->G(s->o_w4),
+                                      as<__nv_bfloat16>(s->dz3), s->G(s->o_w4),
                                       s->G(s->o_b3), c->stream);
     count_launch();
     if (e) return fail(ICP_ERR_DEVICE, "head backward launch failed (%d)", e);
-    // the weight-gradient GEMMs have M = H <= 256 rows, which one CTA covers (two row tiles share
-    // each B chunk): one CTA per SM, each over an equal share of the batch's rows
+    // a weight gradient is one accumulator set of one CTA: one CTA per SM, each over an equal share of
+    // the batch's rows
     const uint32_t splits = std::max<uint32_t>(1u, (uint32_t)c->sms);
     // dW3 = dz3^T h2
     mlp::GemmArgs g = layer(Hn, Hn, (uint32_t)M);
     g.out_f32 = s->G(s->o_w3);
     g.ld_out = Hn;
-    ICP_TRY(run_gemm(s, s->dz3T.ptr, s->h2T.ptr, g, mlp::kAtomicF32, splits));
+    ICP_TRY(run_weight_grad(s, s->dz3.ptr, s->h2.ptr, g, splits));
     // dz2 = (dz3 W3) * silu'(z2), db2
     g = layer(M, Hn, Hn);
     g.z_prev = as<__nv_bfloat16>(s->z2);
     g.out_dz = as<__nv_bfloat16>(s->dz2);
-    g.out_dzT = as<__nv_bfloat16>(s->dz2T);
     g.out_db = s->G(s->o_b2);
     ICP_TRY(run_gemm(s, s->dz3.ptr, s->w3t(), g, mlp::kBackprop, 1));
     // dW2 = dz2^T h1
     g = layer(Hn, Hn, (uint32_t)M);
     g.out_f32 = s->G(s->o_w2);
     g.ld_out = Hn;
-    ICP_TRY(run_gemm(s, s->dz2T.ptr, s->h1T.ptr, g, mlp::kAtomicF32, splits));
-    // dz1 = (dz2 W2) * silu'(z1), db1 (only the column-major copy is read afterwards)
+    ICP_TRY(run_weight_grad(s, s->dz2.ptr, s->h1.ptr, g, splits));
+    // dz1 = (dz2 W2) * silu'(z1), db1 
     g = layer(M, Hn, Hn);
     g.z_prev = as<__nv_bfloat16>(s->z1);
-    g.out_dzT = as<__nv_bfloat16>(s->dz1T);
+    g.out_dz = as<__nv_bfloat16>(s->dz1);
     g.out_db = s->G(s->o_b1);
     ICP_TRY(run_gemm(s, s->dz2.ptr, s->w2t(), g, mlp::kBackprop, 1));
     // dW1 = dz1^T X
     g = layer(Hn, s->K0, (uint32_t)M);
     g.out_f32 = s->G(s->o_w1);
     g.ld_out = s->K0;
-    return run_gemm(s, s->dz1T.ptr, s->XT.ptr, g, mlp::kAtomicF32, splits);
+    return run_weight_grad(s, s->dz1.ptr, s->X.ptr, g, splits);
 }
 
 int refresh_weights(icp_surrogate* s)
@@ -404,7 +403,7 @@ int gradient_pass(icp_surrogate* s, const icp_drop_item* items, uint32_t count, 
 {
     ICP_TRY(begin(s));
     ICP_CUDA(s->y.ensure(4 * (uint64_t)count * s->C));
-    ICP_TRY(enqueue_features(s, items, count, true));
+    ICP_TRY(enqueue_features(s, items, count));
     ICP_TRY(enqueue_forward(s, count, true, as<float>(s->y), nullptr));
     ICP_TRY(enqueue_loss(s, count, d_target));
     return enqueue_backward(s, count);
@@ -546,21 +545,16 @@ int icp_surrogate_create(icp_context* c, const icp_surrogate_config* g, icp_surr
         delete s;
         return st;
     }
-    // the column-major copy of the cell table follows the row-major one
-    std::vector<uint16_t> both(2 * cells.size());
-    std::memcpy(both.data(), cells.data(), 2 * cells.size());
-    for (size_t m = 0; m < s->C; ++m)
-        for (size_t k = 0; k < kc; ++k) both[cells.size() + k * s->C + m] = cells[m * kc + k];
     const size_t np4 = 4 * s->n_params;
     cudaError_t e = cudaSuccess;
     Scratch* p4[] = {&s->params, &s->grads, &s->adam_m, &s->adam_v};
     for (Scratch* x : p4)
         if (e == cudaSuccess) e = x->ensure(np4);
     if (e == cudaSuccess) e = s->wbf.ensure(2 * ((size_t)Hn * s->K0 + 4ull * Hn * Hn));
-    if (e == cudaSuccess) e = s->cells.ensure(2 * both.size());
+    if (e == cudaSuccess) e = s->cells.ensure(2 * cells.size());
     if (e == cudaSuccess) e = s->edges.ensure(sizeof(double) * edges.size());
     if (e == cudaSuccess) e = s->loss.ensure(sizeof(double) * s->R);
-    if (e == cudaSuccess) e = cudaMemcpy(s->cells.ptr, both.data(), 2 * both.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(s->cells.ptr, cells.data(), 2 * cells.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && mlp::fused_shape(s->K0, Hn)) {
         // the cell table in the layout of the input rows (record columns zero), which the fused
         // inference pass loads by TMA before it writes each row's record and axis columns
@@ -676,7 +670,7 @@ int icp_surrogate_predict(icp_surrogate* s, const icp_drop_item* items, uint32_t
     ICP_TRY(check_call(s, items, count));
     if (!d_logits) return fail(ICP_ERR_INVALID_ARGUMENT, "surrogate: null output");
     ICP_TRY(begin(s));
-    ICP_TRY(enqueue_features(s, items, count, false, !fused_inference(s)));
+    ICP_TRY(enqueue_features(s, items, count, !fused_inference(s)));
     ICP_TRY(enqueue_forward(s, count, false, d_logits, nullptr));
     return finish(s->c, "icp_surrogate_predict");
 }
@@ -703,7 +697,7 @@ int icp_surrogate_generate(icp_surrogate* s, const icp_drop_item* items, uint32_
     ICP_CUDA(s->dfrac.ensure(sizeof(double) * s->R * g.nt));
     ICP_CUDA(s->drows.ensure(sizeof(double) * s->R * g.nt));
     ICP_CUDA(cudaMemsetAsync(s->mass_sum.ptr, 0, sizeof(double) * count, c->stream));
-    ICP_TRY(enqueue_features(s, items, count, false, !fused_inference(s)));
+    ICP_TRY(enqueue_features(s, items, count, !fused_inference(s)));
     ICP_TRY(enqueue_forward(s, count, false, nullptr, as<double>(s->mass), as<double>(s->mass_sum)));
     // the analytic diffraction rows on host threads while the device runs the network, into
     // page-locked staging so that the copy, the row scaling, the CDF build and the reports are
@@ -765,7 +759,7 @@ int icp_surrogate_inputs(icp_surrogate* s, const icp_drop_item* items, uint32_t 
     ICP_TRY(check_call(s, items, count));
     if (!h_out) return fail(ICP_ERR_INVALID_ARGUMENT, "surrogate: null output");
     ICP_TRY(begin(s));
-    ICP_TRY(enqueue_features(s, items, count, false));
+    ICP_TRY(enqueue_features(s, items, count));
     ICP_CUDA(cudaMemcpyAsync(h_out, s->X.ptr, 2 * (size_t)count * s->C * s->K0, cudaMemcpyDeviceToHost, s->c->stream));
     return finish(s->c, "icp_surrogate_inputs");
 }
@@ -802,7 +796,6 @@ int icp_mlp_gemm_bf16(icp_context* c, const void* d_a, const void* d_b, uint32_t
     g.K = k;
     g.out_f32 = d_c;
     g.ld_out = n;
-    g.ld_t = m;
     g.error = (unsigned*)c->mlp_error.ptr;
     g.wait_limit = c->wait_limit;
     const int e = mlp::gemm(d_a, d_b, g, accumulate ? mlp::kAtomicF32 : mlp::kStoreF32, split_k ? split_k : 1,

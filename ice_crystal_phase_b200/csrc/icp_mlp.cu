@@ -45,44 +45,6 @@ __global__ void features_kernel(const uint4* __restrict__ rec16, const uint4* __
     }
 }
 
-// XT[k][m]: thread per 8 consecutive rows m of one column k.
-__global__ void features_t_kernel(const __nv_bfloat16* __restrict__ rec16, const uint4* __restrict__ cellsT, uint32_t C,
-                                  uint32_t K0, uint32_t P, uint32_t records, const double* __restrict__ recgeo,
-                                  const double* __restrict__ cellgeo, __nv_bfloat16* __restrict__ XT)
-{
-    const uint64_t per_k = (uint64_t)records * C / 8u;
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= per_k * K0) return;
-    const uint32_t k = (uint32_t)(t / per_k);
-    const uint64_t m8 = t - (uint64_t)k * per_k;
-    const uint64_t m = 8u * m8;
-    const uint32_t r = (uint32_t)(m / C), c = (uint32_t)(m - (uint64_t)r * C);
-    uint4 v;
-    if (k < 16) {
-        const __nv_bfloat16 x = rec16[16u * r + k];
-        const uint32_t w = (uint32_t)__bfloat16_as_ushort(x) * 0x10001u;
-        v = make_uint4(w, w, w, w);
-    } else if (k < K0 - P) {
-        v = cellsT[((uint64_t)(k - 16) * C + c) / 8u];
-    } else {
-        // harmonic j of 8 consecutive cells of one record (C is a multiple of 8)
-        const uint32_t j = k - (K0 - P) + 1u;
-        __align__(16) __nv_bfloat16 h[8];
-        for (int i = 0; i < 8; ++i) {
-            const double x = cos_psi(recgeo, cellgeo, r, c + (uint32_t)i);
-            double tm = 1.0, tt = x;
-            for (uint32_t n = 1; n < j; ++n) {
-                const double tn = __dsub_rn(__dmul_rn(__dmul_rn(2.0, x), tt), tm);
-                tm = tt;
-                tt = tn;
-            }
-            h[i] = __float2bfloat16_rn(__double2float_rn(tt));
-        }
-        v = *reinterpret_cast<const uint4*>(h);
-    }
-    reinterpret_cast<uint4*>(XT + (uint64_t)k * records * C)[m8] = v;
-}
-
 __device__ __forceinline__ double block_sum(double v, double* sh)
 {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -151,20 +113,16 @@ __global__ void __launch_bounds__(1024) softmax_loss_kernel(const float* __restr
 }
 
 // One block of 256 threads per tile of kHeadRows = 64 rows x H columns (H <= 256, a multiple of
-// 64).  Load: thread t owns the 8 columns 8 (t mod H/8) .. and the rows t / (H/8) + k (256 / (H/8)),
-// reading z3 and writing dz3 as 16-byte vectors (coalesced rows); dz3 also goes into a shared
-// tile.  Transpose: thread t < H writes the 64 rows of column t of the tile to dz3T as eight
-// 16-byte vectors (one contiguous 128-byte run per column).  Column sums of dy h3 (dw4) and of
-// dz3 (db3) are reduced in registers and shared memory, one atomic per column per block.
+// 64): thread t owns the 8 columns 8 (t mod H/8) .. and the rows t / (H/8) + k (256 / (H/8)), reading
+// z3 and writing dz3 as 16-byte vectors (coalesced rows); the loads of eight rows are issued together.
+// Column sums of dy h3 (dw4) and of dz3 (db3) are reduced in registers and shared memory, one
+// atomic per column per block.
 constexpr uint32_t kHeadRows = 64;
 __global__ void __launch_bounds__(256) head_backward_kernel(const __nv_bfloat16* __restrict__ z3,
                                                             const float* __restrict__ dy, const float* __restrict__ w4,
                                                             uint32_t M, uint32_t H, __nv_bfloat16* __restrict__ dz3,
-                                                            __nv_bfloat16* __restrict__ dz3T, float* __restrict__ dw4,
-                                                            float* __restrict__ db3)
+                                                            float* __restrict__ dw4, float* __restrict__ db3)
 {
-    // rows are written and columns read contiguously across a warp: no padding needed
-    __shared__ __align__(16) __nv_bfloat16 tile[kHeadRows][256];
     // partial column sums of each row group r0 (rstep groups x H columns = 2048 values for every
     // H): written once per thread, summed in order by one thread per column (no atomics)
     __shared__ float pw[2048], pb[2048];
@@ -174,26 +132,38 @@ __global__ void __launch_bounds__(256) head_backward_kernel(const __nv_bfloat16*
     float w[8], aw[8] = {}, ab[8] = {};
 #pragma unroll
     for (int k = 0; k < 8; ++k) w[k] = w4[c + k];
-    for (uint32_t r = r0; r < kHeadRows; r += rstep) {
-        const uint64_t m = m0 + r;
-        const float d = dy[m];
-        const uint4 u = *reinterpret_cast<const uint4*>(z3 + m * H + c);
-        const uint32_t zw[4] = {u.x, u.y, u.z, u.w};
-        uint32_t ow[4];
+    // H = 256: one pass of eight rows; smaller H: fewer rows per thread, a pass of the same kind
+    for (uint32_t rb = r0; rb < kHeadRows; rb += 8u * rstep) {
+        uint4 zz[8];
+        float dd[8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&zw[q]));
-            const float g0 = d * w[2 * q] * silu_grad_of(z.x), g1 = d * w[2 * q + 1] * silu_grad_of(z.y);
-            aw[2 * q] = fmaf(d, silu_of(z.x), aw[2 * q]);
-            aw[2 * q + 1] = fmaf(d, silu_of(z.y), aw[2 * q + 1]);
-            ab[2 * q] += g0;
-            ab[2 * q + 1] += g1;
-            const __nv_bfloat162 p = __floats2bfloat162_rn(g0, g1);
-            ow[q] = *reinterpret_cast<const uint32_t*>(&p);
+        for (uint32_t i = 0; i < 8; ++i) {
+            const uint32_t r = rb + i * rstep;
+            if (r < kHeadRows) {
+                zz[i] = __ldg(reinterpret_cast<const uint4*>(z3 + (m0 + r) * H + c));
+                dd[i] = __ldg(dy + m0 + r);
+            }
         }
-        const uint4 o = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-        *reinterpret_cast<uint4*>(dz3 + m * H + c) = o;
-        *reinterpret_cast<uint4*>(&tile[r][c]) = o;
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) {
+            const uint32_t r = rb + i * rstep;
+            if (r >= kHeadRows) break;
+            const float d = dd[i];
+            const uint32_t zw[4] = {zz[i].x, zz[i].y, zz[i].z, zz[i].w};
+            uint32_t ow[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&zw[q]));
+                const float g0 = d * w[2 * q] * silu_grad_of(z.x), g1 = d * w[2 * q + 1] * silu_grad_of(z.y);
+                aw[2 * q] = fmaf(d, silu_of(z.x), aw[2 * q]);
+                aw[2 * q + 1] = fmaf(d, silu_of(z.y), aw[2 * q + 1]);
+                ab[2 * q] += g0;
+                ab[2 * q + 1] += g1;
+                const __nv_bfloat162 p = __floats2bfloat162_rn(g0, g1);
+                ow[q] = *reinterpret_cast<const uint32_t*>(&p);
+            }
+            *reinterpret_cast<uint4*>(dz3 + (m0 + r) * H + c) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+        }
     }
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -202,14 +172,6 @@ __global__ void __launch_bounds__(256) head_backward_kernel(const __nv_bfloat16*
     }
     __syncthreads();
     if (t < H) {
-        __nv_bfloat16* dst = dz3T + (uint64_t)t * M + m0;
-#pragma unroll
-        for (uint32_t r8 = 0; r8 < kHeadRows; r8 += 8) {
-            __align__(16) __nv_bfloat16 col[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) col[k] = tile[r8 + k][t];
-            *reinterpret_cast<uint4*>(dst + r8) = *reinterpret_cast<const uint4*>(col);
-        }
         float sw = 0.0f, sb = 0.0f;
         for (uint32_t k = 0; k < rstep; ++k) {
             sw += pw[k * H + t];
@@ -279,8 +241,7 @@ unsigned blocks_of(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t);
 } // namespace
 
 int launch_features(const __nv_bfloat16* rec16, const __nv_bfloat16* cells, uint32_t records, uint32_t C, uint32_t K0,
-                    uint32_t P, const double* recgeo, const double* cellgeo, __nv_bfloat16* X, __nv_bfloat16* XT,
-                    cudaStream_t st)
+                    uint32_t P, const double* recgeo, const double* cellgeo, __nv_bfloat16* X, cudaStream_t st)
 {
     if (K0 % 64 || C % 128 || !records || P % 8 || P + 16 > K0) return -1;
     const uint32_t q_row = K0 / 8u;
@@ -289,12 +250,6 @@ int launch_features(const __nv_bfloat16* rec16, const __nv_bfloat16* cells, uint
                                                            reinterpret_cast<const uint4*>(cells), C, q_row,
                                                            q_row - P / 8u, total, recgeo, cellgeo,
                                                            reinterpret_cast<uint4*>(X));
-    if (XT) {
-        // the column-major cell table follows the row-major one in the same allocation
-        const uint4* cellsT = reinterpret_cast<const uint4*>(cells + (uint64_t)C * (K0 - 16));
-        const uint64_t n = (uint64_t)records * C / 8u * K0;
-        features_t_kernel<<<blocks_of(n, 256), 256, 0, st>>>(rec16, cellsT, C, K0, P, records, recgeo, cellgeo, XT);
-    }
     return (int)cudaGetLastError();
 }
 
@@ -307,10 +262,10 @@ int launch_softmax_loss(const float* y, const float* p, uint32_t records, uint32
 }
 
 int launch_head_backward(const __nv_bfloat16* z3, const float* dy, const float* w4, uint32_t M, uint32_t H,
-                         __nv_bfloat16* dz3, __nv_bfloat16* dz3T, float* dw4, float* db3, cudaStream_t st)
+                         __nv_bfloat16* dz3, float* dw4, float* db3, cudaStream_t st)
 {
     if (M % kHeadRows || H > 256 || H % 64) return -1;
-    head_backward_kernel<<<M / kHeadRows, 256, 0, st>>>(z3, dy, w4, M, H, dz3, dz3T, dw4, db3);
+    head_backward_kernel<<<M / kHeadRows, 256, 0, st>>>(z3, dy, w4, M, H, dz3, dw4, db3);
     return (int)cudaGetLastError();
 }
 

@@ -3,21 +3,20 @@
 //
 //   D[M x N] = A[M x K] * B[N x K]^T      A, B: BF16, K-major (row-major with K contiguous)
 //
-// Three kernels.  Inference of the default network shape runs as one persistent kernel that takes
+// Four kernels.  Inference of the default network shape runs as one persistent kernel that takes
 // each 128-row tile from its input row to y with the activations on chip (mlp_fused_kernel,
 // below).  The layer GEMMs of training and of other shapes (K, N = layer widths <= 256, M = the
 // rows of a batch) run persistent and warp-specialised (gemm_persistent_kernel).  The weight
-// gradients (M, N =
-// layer widths, K = rows of a batch) run split-K (gemm_kernel): one CTA of 128 threads computes a
+// gradients contract over the rows of a batch (weight_grad_kernel).  Split-K products of K-major
+// operands (icp_mlp_gemm_bf16) run in gemm_kernel: one CTA of 128 threads computes a
 // 128 x N tile (N in {64, 128, 256}) over a range of K chunks of 64: thread 0 streams A and B
 // chunks through a STAGES-deep ring with 2-D TMA loads (128-byte swizzle, completion counted on a
 // "full" mbarrier per stage) and issues four K=16 tcgen05.mma per chunk into an FP32 accumulator
 // in tensor memory; each chunk's MMAs commit to the stage's "empty" mbarrier, which gates the
 // refill.  After the last chunk a commit to "done" releases the epilogue: warp w reads TMEM lanes
-// 32w..32w+31 (rows) with tcgen05.ld, 32 columns at a time, and applies one of the fused
-// epilogues below.  Split-K (grid.y > 1) adds partial tiles with FP32 atomics.  Every mbarrier
-// wait is bounded: on expiry the kernel sets the error word, waits (bounded) for its issued loads
-// and MMAs, frees its tensor memory and returns.
+// 32w..32w+31 (rows) with tcgen05.ld, 32 columns at a time.  Split-K (grid.y > 1) adds partial tiles
+// with FP32 atomics.  Every mbarrier wait is bounded: on expiry the kernel sets the error word,
+// waits (bounded) for its issued loads and MMAs, frees its tensor memory and returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -43,10 +42,10 @@ template <int N, int MT = 1> __host__ __device__ constexpr uint32_t stage_bytes(
 {
     return (uint32_t)MT * kA + (uint32_t)N * 128u;
 }
-// 1024 (alignment) + stages + barriers / TMEM slot (256) + column sums of the bias gradient (1024)
+// 1024 (alignment) + stages + barriers / TMEM slot (256)
 template <int N, int MT = 1> constexpr size_t smem_bytes()
 {
-    return 1024 + (size_t)stages<N, MT>() * stage_bytes<N, MT>() + 256 + 1024;
+    return 1024 + (size_t)stages<N, MT>() * stage_bytes<N, MT>() + 256;
 }
 
 // Logistic function 1 / (1 + exp(-z)) with the exponential on the special-function unit and
@@ -87,20 +86,6 @@ template <bool kFmaRcp> __device__ __forceinline__ float silu_grad(float z)
     return s * (1.0f + z * (1.0f - s));
 }
 
-__device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const float (&v)[32])
-{
-    uint4* d = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        uint32_t w[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __nv_bfloat162 p = __floats2bfloat162_rn(v[8 * q + 2 * i], v[8 * q + 2 * i + 1]);
-            w[i] = *reinterpret_cast<const uint32_t*>(&p);
-        }
-        d[q] = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-}
 // Column sums of a warp's 32 x 32 block (lane = row, v[i] = column i): a butterfly
 // reduce-scatter in 31 shuffles, after which lane L holds the sum of column L in v[0].
 __device__ __forceinline__ float warp_column_sum(float (&v)[32], uint32_t lane)
@@ -118,123 +103,154 @@ __device__ __forceinline__ float warp_column_sum(float (&v)[32], uint32_t lane)
     return v[0];
 }
 
-// Column-major copy of a warp's 32 rows x 32 columns through the warp's shared transpose buffer
-// (32 rows of 40 BF16, 80-byte stride): lane L writes its row, then gathers column L and writes
-// its 32 rows (64 contiguous bytes) to dst_col0 + L * ld with four 16-byte stores.  dst_col0 is
-// the column's first row of this warp (32-row aligned).  Every index is a compile-time constant.
-constexpr uint32_t kTStride = 40; // BF16 per transpose-buffer row
-__device__ __forceinline__ void store_bf16x32_t(__nv_bfloat16* dst_col0, uint32_t ld, const float (&v)[32],
-                                                __nv_bfloat16* tbuf, uint32_t lane)
+// A warp's tile of 32 rows x 64 BF16 columns between its row-per-lane form (lane = row, w[32] its 64
+// values) and global memory, through 4 KB of shared memory with the 16-byte chunks of row r
+// exchanged by r mod 8 (no bank conflicts either way): every global access then covers four whole
+// 128-byte lines, where a row per lane touches 32 half-used sectors (with the column-major copies
+// that the weight gradients read before: 1.92 ms per hidden layer of 16 records, 0.52 .. 0.60 now).
+constexpr uint32_t kTileBytes = 32u * 128u;
+__device__ __forceinline__ uint4* tile_chunk(uint8_t* buf, uint32_t row, uint32_t ch)
 {
-    uint4* row = reinterpret_cast<uint4*>(tbuf + lane * kTStride);
+    return reinterpret_cast<uint4*>(buf + row * 128u + ((ch ^ (row & 7u)) << 4));
+}
+__device__ __forceinline__ void store_tile(__nv_bfloat16* dst, uint32_t ld, const uint32_t (&w)[32], uint8_t* buf,
+                                           uint32_t lane)
+{
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        uint32_t w[4];
+    for (uint32_t ch = 0; ch < 8; ++ch)
+        *tile_chunk(buf, lane, ch) = make_uint4(w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
+    __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __nv_bfloat162 p = __floats2bfloat162_rn(v[8 * q + 2 * i], v[8 * q + 2 * i + 1]);
-            w[i] = *reinterpret_cast<const uint32_t*>(&p);
-        }
-        row[q] = make_uint4(w[0], w[1], w[2], w[3]);
+    for (uint32_t i = 0; i < 8; ++i) {
+        const uint32_t row = 4u * i + (lane >> 3), ch = lane & 7u;
+        *reinterpret_cast<uint4*>(dst + (size_t)row * ld + 8u * ch) = *tile_chunk(buf, row, ch);
     }
     __syncwarp();
-    const uint16_t* col = reinterpret_cast<const uint16_t*>(tbuf) + lane;
-    uint32_t w[16];
+}
+// This lane's share of a tile (issued early; the values land in `part`), then the row-per-lane form.
+__device__ __forceinline__ void load_tile(const __nv_bfloat16* src, uint32_t ld, uint32_t lane, uint4 (&part)[8])
+{
 #pragma unroll
-    for (int r = 0; r < 16; ++r)
-        w[r] = (uint32_t)col[(2 * r) * kTStride] | ((uint32_t)col[(2 * r + 1) * kTStride] << 16);
-    uint4* d = reinterpret_cast<uint4*>(dst_col0 + (size_t)lane * ld);
+    for (uint32_t i = 0; i < 8; ++i)
+        part[i] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(4u * i + (lane >> 3)) * ld + 8u * (lane & 7u)));
+}
+__device__ __forceinline__ void tile_rows(const uint4 (&part)[8], uint8_t* buf, uint32_t lane, uint32_t (&w)[32])
+{
 #pragma unroll
-    for (int q = 0; q < 4; ++q) d[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+    for (uint32_t i = 0; i < 8; ++i) *tile_chunk(buf, 4u * i + (lane >> 3), lane & 7u) = part[i];
+    __syncwarp();
+#pragma unroll
+    for (uint32_t ch = 0; ch < 8; ++ch) {
+        const uint4 u = *tile_chunk(buf, lane, ch);
+        w[4 * ch] = u.x;
+        w[4 * ch + 1] = u.y;
+        w[4 * ch + 2] = u.z;
+        w[4 * ch + 3] = u.w;
+    }
     __syncwarp();
 }
-
-__device__ __forceinline__ void load_bf16x32(const __nv_bfloat16* src, float (&v)[32])
+__device__ __forceinline__ void pack_bf16(const float (&v)[2][32], uint32_t (&w)[32])
 {
-    const uint4* s = reinterpret_cast<const uint4*>(src);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint4 u = s[q];
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __nv_bfloat162 p = *reinterpret_cast<const __nv_bfloat162*>(&w[i]);
-            const float2 f = __bfloat1622float2(p);
-            v[8 * q + 2 * i] = f.x;
-            v[8 * q + 2 * i + 1] = f.y;
+        for (int i = 0; i < 16; ++i) {
+            const __nv_bfloat162 p = __floats2bfloat162_rn(v[h][2 * i], v[h][2 * i + 1]);
+            w[16 * h + i] = *reinterpret_cast<const uint32_t*>(&p);
         }
-    }
 }
 
-// Columns [c0, c1) of one row of a 128 x N accumulator tile through the fused epilogue: this
-// thread's TMEM lane starts at taddr (column 0); m is the output row; bias / head_w point at N
-// values (shared or global memory, 16-byte aligned); colsum collects the bias gradient
-// (kBackprop).  Returns the partial head sum of these columns (kHead).
-template <int N, int EPI>
-__device__ __forceinline__ float epilogue_cols(const GemmArgs& g, uint32_t taddr, uint32_t m, uint32_t lane,
-                                              uint32_t c0, uint32_t c1, const float* bias, const float* head_w,
-                                              float* colsum, __nv_bfloat16* tbuf)
+// Columns [0, N) of one row of a 128 x N accumulator tile to FP32 (kStoreF32, kAtomicF32): this
+// thread's TMEM lane starts at taddr, m is the output row.
+template <int EPI>
+__device__ __forceinline__ void epilogue_f32(const GemmArgs& g, uint32_t taddr, uint32_t m, uint32_t c0, uint32_t c1)
 {
-    constexpr bool kHeadEpi = EPI == kHead || EPI == kHeadTrain;
-    constexpr bool kTrain = EPI == kHiddenTrain || EPI == kHeadTrain;
-    constexpr bool kLayer = kHeadEpi || EPI == kHidden || EPI == kHiddenTrain;
-    float yacc = 0.0f;
-    // columns in pairs of 32: both TMEM loads of a pair are in flight together (one wait per 64
-    // columns; c1 - c0 is a multiple of 64)
 #pragma unroll 1
-    for (uint32_t c2 = c0; c2 < c1; c2 += 64u) {
-        float vv[2][32];
-        umma::tmem_ld32x2(taddr + c2, vv[0], vv[1]);
-#pragma unroll
-    for (uint32_t h = 0; h < 2; ++h) { // unrolled: vv[h] stays in registers
-        const uint32_t c = c2 + 32u * h;
-        float (&v)[32] = vv[h];
+    for (uint32_t c = c0; c < c1; c += 32u) {
+        float v[32];
+        umma::tmem_ld32(taddr + c, v);
         if constexpr (EPI == kStoreF32) {
             float4* d = reinterpret_cast<float4*>(g.out_f32 + (size_t)m * g.ld_out + c);
 #pragma unroll
             for (int q = 0; q < 8; ++q) d[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        } else if constexpr (EPI == kAtomicF32) {
+        } else {
             float* d = g.out_f32 + (size_t)m * g.ld_out + c;
 #pragma unroll
             for (int i = 0; i < 32; ++i) atomicAdd(d + i, v[i]);
-        } else if constexpr (kLayer) {
+        }
+    }
+}
+
+// Columns [c0, c1) (a multiple of 64) of a warp's 32 rows m0 .. m0 + 31 of a 128 x N accumulator tile
+// through a layer's epilogue: this thread's TMEM lane starts at taddr (column 0), its row is m0 + lane;
+// bias / head_w point at N values (16-byte aligned); colsum collects the bias gradient and z holds
+// the first 64 columns of z_prev already requested with load_tile (kBackprop); buf is the warp's tile
+// buffer.  Returns the partial head sum of these columns (kHead).
+template <int N, int EPI>
+__device__ __forceinline__ float epilogue_layer(const GemmArgs& g, uint32_t taddr, uint32_t m0, uint32_t lane,
+                                                uint32_t c0, uint32_t c1, const float* bias, const float* head_w,
+                                                float* colsum, uint4 (&z)[8], uint8_t* buf)
+{
+    constexpr bool kHeadEpi = EPI == kHead || EPI == kHeadTrain;
+    constexpr bool kTrain = EPI == kHiddenTrain || EPI == kHeadTrain;
+    float yacc = 0.0f;
+#pragma unroll 1
+    for (uint32_t c = c0; c < c1; c += 64u) {
+        float v[2][32];
+        umma::tmem_ld32x2(taddr + c, v[0], v[1]); // both loads in flight, one wait
+        uint32_t w[32];
+        if constexpr (EPI == kBackprop) {
+            tile_rows(z, buf, lane, w);
+            if (c + 64u < c1) load_tile(g.z_prev + (size_t)m0 * N + c + 64u, N, lane, z);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[16 * h + i]));
+                    v[h][2 * i] *= silu_grad<false>(f.x);
+                    v[h][2 * i + 1] *= silu_grad<false>(f.y);
+                }
+            pack_bf16(v, w);
+            store_tile(g.out_dz + (size_t)m0 * N + c, N, w, buf, lane);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) atomicAdd(&colsum[c + 32u * h + lane], warp_column_sum(v[h], lane));
+        } else {
             const float4* b4 = reinterpret_cast<const float4*>(bias + c);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
+            for (int q = 0; q < 16; ++q) {
                 const float4 b = b4[q];
-                v[4 * q] += b.x;
-                v[4 * q + 1] += b.y;
-                v[4 * q + 2] += b.z;
-                v[4 * q + 3] += b.w;
+                float* x = &v[q / 8][4 * (q % 8)];
+                x[0] += b.x;
+                x[1] += b.y;
+                x[2] += b.z;
+                x[3] += b.w;
             }
             if constexpr (kTrain)
-                if (g.out_z) store_bf16x32(g.out_z + (size_t)m * N + c, v);
+                if (g.out_z) {
+                    pack_bf16(v, w);
+                    store_tile(g.out_z + (size_t)m0 * N + c, N, w, buf, lane);
+                }
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = silu<!kTrain>(v[i]);
-            if (g.out_h) store_bf16x32(g.out_h + (size_t)m * N + c, v);
-            if constexpr (kTrain)
-                if (g.out_hT) store_bf16x32_t(g.out_hT + (size_t)c * g.ld_t + (m - lane), g.ld_t, v, tbuf, lane);
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[h][i] = silu<!kTrain>(v[h][i]);
+            if (g.out_h) {
+                pack_bf16(v, w);
+                store_tile(g.out_h + (size_t)m0 * N + c, N, w, buf, lane);
+            }
             if constexpr (kHeadEpi) {
                 const float4* w4 = reinterpret_cast<const float4*>(head_w + c);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const float4 w = w4[q];
-                    yacc = fmaf(v[4 * q], w.x, yacc);
-                    yacc = fmaf(v[4 * q + 1], w.y, yacc);
-                    yacc = fmaf(v[4 * q + 2], w.z, yacc);
-                    yacc = fmaf(v[4 * q + 3], w.w, yacc);
+                for (int q = 0; q < 16; ++q) {
+                    const float4 hw = w4[q];
+                    const float* x = &v[q / 8][4 * (q % 8)];
+                    yacc = fmaf(x[0], hw.x, yacc);
+                    yacc = fmaf(x[1], hw.y, yacc);
+                    yacc = fmaf(x[2], hw.z, yacc);
+                    yacc = fmaf(x[3], hw.w, yacc);
                 }
             }
-        } else if constexpr (EPI == kBackprop) {
-            float z[32];
-            load_bf16x32(g.z_prev + (size_t)m * N + c, z);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] *= silu_grad<false>(z[i]);
-            if (g.out_dz) store_bf16x32(g.out_dz + (size_t)m * N + c, v);
-            if (g.out_dzT) store_bf16x32_t(g.out_dzT + (size_t)c * g.ld_t + (m - lane), g.ld_t, v, tbuf, lane);
-            if (g.out_db) atomicAdd(&colsum[c + lane], warp_column_sum(v, lane));
         }
-    }
     }
     return yacc;
 }
@@ -256,8 +272,7 @@ __device__ __forceinline__ void head_store(const GemmArgs& g, uint32_t m, float 
     }
 }
 
-// Split-K GEMM (one 128-row tile and one K range per CTA): the weight gradients, whose K (the
-// rows of a batch) is long and whose M and N are the layer widths.
+// Split-K GEMM (one 128-row tile and one K range per CTA) of K-major operands.
 template <int N, int EPI, int MT = 1>
 __global__ void __launch_bounds__(128, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g)
@@ -272,10 +287,8 @@ __global__ void __launch_bounds__(128, 1)
     uint64_t* done = empty + S;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
-    float* colsum = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(full) + 256);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    if constexpr (EPI == kBackprop)
-        for (uint32_t i = threadIdx.x; i < (uint32_t)N; i += blockDim.x) colsum[i] = 0.0f;
+    static_assert(EPI == kStoreF32 || EPI == kAtomicF32, "the layers run persistent");
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
@@ -352,20 +365,10 @@ __global__ void __launch_bounds__(128, 1)
     const bool ready = __all_sync(0xffffffffu, mine && !*abort_flag);
     umma::fence_after_sync();
     if (ready) {
-        // the stages are free once every MMA has completed: one transpose buffer per warp there
-        __nv_bfloat16* tbuf = reinterpret_cast<__nv_bfloat16*>(smem) + (size_t)warp * 32u * kTStride;
 #pragma unroll 1
-        for (int mt = 0; mt < MT; ++mt) {
-            const uint32_t m = m0 + 128u * mt + 32u * warp + lane;
-            const float y = epilogue_cols<N, EPI>(g, tmem + ((32u * warp) << 16) + (uint32_t)(mt * N), m, lane, 0u,
-                                                  (uint32_t)N, g.bias, g.head_w, colsum, tbuf);
-            if constexpr (EPI == kHead || EPI == kHeadTrain) head_store(g, m, y);
-        }
-    }
-    if constexpr (EPI == kBackprop) {
-        __syncthreads();
-        if (g.out_db && ready)
-            for (uint32_t i = threadIdx.x; i < (uint32_t)N; i += blockDim.x) atomicAdd(&g.out_db[i], colsum[i]);
+        for (int mt = 0; mt < MT; ++mt)
+            epilogue_f32<EPI>(g, tmem + ((32u * warp) << 16) + (uint32_t)(mt * N), m0 + 128u * mt + 32u * warp + lane,
+                              0u, (uint32_t)N);
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -391,7 +394,7 @@ constexpr uint32_t kSlices = kEpiWarps / 4;
 constexpr uint32_t kPThreads = 64 + 32 * kEpiWarps;
 // per-CTA extras after the ring: barriers (1 KB), colsum, bias, head weights (1 KB each), head
 // partial sums (kSlices - 1 slices x 128 floats, rounded up to kSlices)
-constexpr int kPExtra = 1024 + 3 * 1024 + (int)kSlices * 512 + (int)(kEpiWarps * 32u * kTStride * 2u);
+constexpr int kPExtra = 1024 + 3 * 1024 + (int)kSlices * 512 + (int)(kEpiWarps * kTileBytes);
 template <int N, int KC> __host__ __device__ constexpr int pstages()
 {
     return (232448 - 1024 - N * 128 * KC - kPExtra) / (int)kA > 8 ? 8
@@ -434,7 +437,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
     float* sbias = colsum + 256;
     float* shead = sbias + 256;
     float* ypart = shead + 256; // [kSlices - 1][128]
-    __nv_bfloat16* tbufs = reinterpret_cast<__nv_bfloat16*>(ypart + kSlices * 128u); // per epilogue warp
+    uint8_t* tbufs = reinterpret_cast<uint8_t*>(ypart + kSlices * 128u); // per epilogue warp
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t tiles = g.M / 128u;
 
@@ -539,11 +542,14 @@ __global__ void __launch_bounds__(kPThreads, 1)
         const uint32_t q = warp & 3u, slice = (warp - 2u) >> 2;
         const uint32_t c0 = slice * W;
         const uint32_t row = 32u * q + lane;
+        uint8_t* buf = tbufs + (warp - 2u) * kTileBytes;
         uint32_t i = 0;
         bool live = true;
 #pragma unroll 1
         for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
             const uint32_t b = i & 1u;
+            uint4 z[8]; // requested before the accumulator is waited for
+            if constexpr (EPI == kBackprop) load_tile(g.z_prev + (size_t)(t * 128u + 32u * q) * N + c0, N, lane, z);
             const bool mine = live && umma::mbar_wait(&acc_full[b], (i >> 1) & 1u, kWaitLimit);
             if (!__all_sync(0xffffffffu, mine && !*abort_flag)) {
                 if (lane == 0 && live) {
@@ -555,8 +561,11 @@ __global__ void __launch_bounds__(kPThreads, 1)
             float y = 0.0f;
             if (live) {
                 umma::fence_after_sync();
-                y = epilogue_cols<N, EPI>(g, tmem + ((32u * q) << 16) + b * (uint32_t)N, t * 128u + row, lane, c0,
-                                          c0 + W, sbias, shead, colsum, tbufs + (warp - 2u) * 32u * kTStride);
+                const uint32_t taddr = tmem + ((32u * q) << 16) + b * (uint32_t)N;
+                if constexpr (EPI == kStoreF32) epilogue_f32<EPI>(g, taddr, t * 128u + row, c0, c0 + W);
+                else
+                    y = epilogue_layer<N, EPI>(g, taddr, t * 128u + 32u * q, lane, c0, c0 + W, sbias, shead, colsum, z,
+                                               buf);
                 umma::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) umma::mbar_arrive(&acc_empty[b]);
@@ -694,6 +703,158 @@ bool persistent_shape(const GemmArgs& g)
 {
     const uint32_t kc = g.K / 64u;
     return (g.N == 128 || g.N == 256) && (kc == 1 || kc == 2 || kc == 4);
+}
+
+// ---------------------------------------------------------------- weight gradients
+// D[128 MT x N] += A^T B over a range of rows (A [rows x 128 MT], B [rows x N], row-major BF16): the
+// contraction runs over the rows, so both operands are MN-major as they lie and no transposed copy of
+// an activation exists.  One CTA holds the whole gradient in tensor memory and takes an equal share of
+// the batch's rows: warp 0 streams 64-row chunks with TMA (boxes of 64 columns x 64 rows, 128-byte
+// swizzle) through a ring of 64 KB stages (N = 256), one thread of warp 1 issues four K=16 steps per
+// chunk and row tile, and after the last chunk warps 2..5 add the tile to memory with four-wide
+// FP32 reductions.  Bound by the reads of A and B (2.1 GB for 16 records of 131072 rows, 0.33 ms at the
+// measured rate): 0.33 ms; from column-major copies, one thread loading, issuing and waiting in
+// turn and scalar atomics, 0.90 ms, and the copies cost the layers as much again.
+constexpr uint32_t kBox = 64u * 128u; // bytes of a 64-column x 64-row box
+template <int N, int MT> __host__ __device__ constexpr uint32_t wg_stage() { return (2u * MT + (uint32_t)N / 64u) * kBox; }
+template <int N, int MT> __host__ __device__ constexpr int wg_stages()
+{
+    return (int)((232448u - 2048u) / wg_stage<N, MT>()) > 6 ? 6 : (int)((232448u - 2048u) / wg_stage<N, MT>());
+}
+constexpr uint32_t kWgThreads = 192;
+
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d)
+{
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
+                 : "memory");
+}
+
+template <int N, int MT>
+__global__ void __launch_bounds__(kWgThreads, 1)
+    weight_grad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                       const GemmArgs g)
+{
+    constexpr int S = wg_stages<N, MT>();
+    constexpr uint32_t SB = wg_stage<N, MT>(), BOFF = 2u * MT * kBox;
+    static_assert(S >= 2, "ring too shallow");
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * SB);
+    uint64_t* empty = full + S;
+    uint64_t* done = empty + S;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S; ++s) {
+            umma::mbar_init(&full[s], 1);
+            umma::mbar_init(&empty[s], 1);
+        }
+        umma::mbar_init(done, 1);
+        *abort_flag = 0;
+        umma::mbar_fence_init();
+    }
+    if (warp == 1) umma::tmem_alloc(tslot, (uint32_t)(MT * N));
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tmem = *tslot;
+    const uint32_t kc0 = blockIdx.x * g.k_chunks, kc1 = min(g.K / 64u, kc0 + g.k_chunks);
+    const uint32_t nk = kc1 > kc0 ? kc1 - kc0 : 0u;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            bool ok = true;
+            uint32_t kc = 0;
+            for (; kc < nk; ++kc) {
+                const uint32_t s = kc % S;
+                if ((kc >= (uint32_t)S && !umma::mbar_wait(&empty[s], ((kc / S) & 1u) ^ 1u, kWaitLimit)) || *abort_flag) {
+                    ok = false;
+                    break;
+                }
+                uint8_t* a = smem + s * SB;
+                const int32_t row = (int32_t)((kc0 + kc) * 64u);
+                umma::mbar_arrive_expect_tx(&full[s], SB);
+#pragma unroll
+                for (int j = 0; j < 2 * MT; ++j) umma::tma_load_2d(a + j * kBox, &tmA, &full[s], 64 * j, row);
+#pragma unroll
+                for (int j = 0; j < N / 64; ++j) umma::tma_load_2d(a + BOFF + j * kBox, &tmB, &full[s], 64 * j, row);
+            }
+            if (!ok) {
+                *abort_flag = 1;
+                atomicExch(g.error, 7u);
+            }
+            // every issued load lands before the CTA's shared memory is released
+            for (uint32_t j = kc > (uint32_t)S ? kc - S : 0u; j < kc; ++j)
+                umma::mbar_wait(&full[j % S], (j / S) & 1u, kWaitLimit);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = umma::instr_desc_bf16_f32_mn(128, (uint32_t)N);
+            bool ok = nk > 0;
+            for (uint32_t kc = 0; kc < nk && ok; ++kc) {
+                const uint32_t s = kc % S;
+                if (!umma::mbar_wait(&full[s], (kc / S) & 1u, kWaitLimit) || *abort_flag) {
+                    ok = false;
+                    break;
+                }
+                umma::fence_after_sync();
+                const uint32_t a = umma::smem_u32(smem + s * SB), b = a + BOFF;
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k)
+                        umma::mma_bf16(tmem + (uint32_t)(mt * N),
+                                       umma::smem_desc_sw128_mn(a + 2u * mt * kBox + 2048u * k, kBox),
+                                       umma::smem_desc_sw128_mn(b + 2048u * k, kBox), idesc, kc > 0 || k > 0);
+                umma::mma_commit(&empty[s]);
+            }
+            if (!ok) {
+                *abort_flag = 1;
+                if (nk) atomicExch(g.error, 8u);
+                __threadfence_block();
+            }
+            umma::mma_commit(done); // arrives once every MMA issued above has completed
+        }
+    } else {
+        const bool mine = umma::mbar_wait(done, 0, kWaitLimit);
+        if (!mine) atomicExch(g.error, 9u);
+        const bool ready = __all_sync(0xffffffffu, mine && !*abort_flag);
+        umma::fence_after_sync();
+        if (ready) {
+            const uint32_t q = warp & 3u;
+#pragma unroll 1
+            for (int mt = 0; mt < MT; ++mt) {
+                float* out = g.out_f32 + (size_t)(128u * mt + 32u * q + lane) * g.ld_out;
+#pragma unroll 1
+                for (uint32_t c = 0; c < (uint32_t)N; c += 32u) {
+                    float v[32];
+                    umma::tmem_ld32(tmem + ((32u * q) << 16) + (uint32_t)(mt * N) + c, v);
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) red_add4(out + c + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
+                }
+            }
+        }
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        // also after an abort: no MMA runs on freed tensor memory
+        umma::mbar_wait(done, 0, kWaitLimit);
+        umma::tmem_dealloc(tmem, (uint32_t)(MT * N));
+    }
+}
+
+template <int N, int MT> int launch_wg(const void* A, const void* B, const GemmArgs& g, uint32_t splits, cudaStream_t st)
+{
+    CUtensorMap ta, tb;
+    if (make_map(&ta, A, g.K, g.M, 64u) || make_map(&tb, B, g.K, (uint32_t)N, 64u)) return -1;
+    const size_t smem = 1024 + (size_t)wg_stages<N, MT>() * wg_stage<N, MT>() + 256;
+    const cudaError_t e =
+        cudaFuncSetAttribute(weight_grad_kernel<N, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    weight_grad_kernel<N, MT><<<splits, kWgThreads, smem, st>>>(ta, tb, g);
+    return (int)cudaGetLastError();
 }
 
 // ---------------------------------------------------------------- fused inference pass
@@ -1158,13 +1319,25 @@ int gemm(const void* A, const void* B, GemmArgs g, int epi, uint32_t splits, cud
     switch (epi) {
     case kStoreF32: return launch_epi<kStoreF32>(A, B, g, splits, st);
     case kAtomicF32: return launch_epi<kAtomicF32>(A, B, g, splits, st);
-    case kHidden: return launch_epi<kHidden>(A, B, g, 1, st);
-    case kHead: return launch_epi<kHead>(A, B, g, 1, st);
-    case kHiddenTrain: return launch_epi<kHiddenTrain>(A, B, g, 1, st);
-    case kHeadTrain: return launch_epi<kHeadTrain>(A, B, g, 1, st);
-    case kBackprop: return launch_epi<kBackprop>(A, B, g, 1, st);
-    default: return -4;
+    default: return -4; // layers have persistent shapes
     }
+}
+
+int weight_grad(const void* A, const void* B, GemmArgs g, uint32_t splits, cudaStream_t st)
+{
+    if (g.K == 0 || g.K % 64u || !splits) return -3;
+    const uint32_t nk = g.K / 64u;
+    g.k_chunks = (nk + splits - 1) / splits;
+    splits = (nk + g.k_chunks - 1) / g.k_chunks;
+    if (g.M == 256u) {
+        if (g.N == 64u) return launch_wg<64, 2>(A, B, g, splits, st);
+        if (g.N == 128u) return launch_wg<128, 2>(A, B, g, splits, st);
+        if (g.N == 256u) return launch_wg<256, 2>(A, B, g, splits, st);
+    } else if (g.M == 128u) {
+        if (g.N == 64u) return launch_wg<64, 1>(A, B, g, splits, st);
+        if (g.N == 128u) return launch_wg<128, 1>(A, B, g, splits, st);
+    }
+    return -2;
 }
 
 bool fused_shape(uint32_t K0, uint32_t H) { return H == 256u && (K0 == 64u || K0 == 128u); }

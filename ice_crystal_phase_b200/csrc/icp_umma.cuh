@@ -29,11 +29,32 @@ __host__ __device__ constexpr uint32_t instr_desc_bf16_f32(uint32_t m, uint32_t 
     return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
+// Instruction descriptor with both operands MN-major (bits 15 and 16): the contraction runs over the
+// rows of the tiles.
+__host__ __device__ constexpr uint32_t instr_desc_bf16_f32_mn(uint32_t m, uint32_t n)
+{
+    return instr_desc_bf16_f32(m, n) | (1u << 15) | (1u << 16);
+}
+
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr)
 {
     uint64_t d = 0;
     d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
     d |= (uint64_t)1u << 16;
+    d |= (uint64_t)(1024u >> 4) << 32;
+    d |= (uint64_t)1u << 46;
+    d |= (uint64_t)2u << 61;
+    return d;
+}
+
+// MN-major tile as a TMA load of {64 columns, rows} leaves it: row k (the contraction index) at byte
+// 128 k, 8-row groups 1024 bytes apart (the stride offset), the next 64 columns `group_bytes` on (the
+// leading offset).  Stepping K by 16 advances the start address by 2048 bytes.
+__device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t saddr, uint32_t group_bytes)
+{
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
+    d |= (uint64_t)(group_bytes >> 4) << 16;
     d |= (uint64_t)(1024u >> 4) << 32;
     d |= (uint64_t)1u << 46;
     d |= (uint64_t)2u << 61;
