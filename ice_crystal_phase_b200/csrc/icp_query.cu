@@ -63,7 +63,10 @@ constexpr unsigned kQueryBlocksPerSm = 6;
 constexpr unsigned kScanThreads = 1024;
 constexpr int kBinRows = 256, kBinCols = 512;
 constexpr double kPi = 3.141592653589793238462643383279502884;
-constexpr double kCapMargin = 1e-4; // radians added to every cap (rounding of the box test)
+// Radians added to every cap: the roundings of the box test move a ray by some 1e-7, those of acos and
+// atan2 by 1e-8 at most (next to a pole).  The bins are those that the widened cap touches and no more: one
+// spare bin on every side put 3 x 3 bins or more under a patch that is a third of a bin wide.
+constexpr double kCapMargin = 1e-4;
 
 // query flags (PatchQueryFlags) and intersector flags (BilinearHitFlags, BilinearQueryFlags)
 enum : uint32_t { qUnresolved = 1, qInvalid = 2, qMismatch = 4, qRefine = 8, qBoundary = 16, qFp64 = 32,
@@ -140,10 +143,16 @@ __device__ __forceinline__ F3 evaluate(const F3* c, float u, float v)
 // The ray w through the origin against the bilinear patch of the four corner directions,
 // in the plane normal to w's dominant axis: a quadratic in u, then three Newton steps.
 // Returns true when the result is not conclusive (the caller retries in binary64).
-template <class T> __device__ bool solve(const F3* corner, F3 dir, Hits& out)
+// The patch in the plane normal to w's dominant axis, scaled: a + b u + c v + d u v.
+template <class T> struct Planar {
+    P3<T> w, p0, p1, p2, p3;
+    P2<T> a, b, c, d;
+    unsigned kz;
+};
+enum Reach { kNoRoot, kMaybeRoot, kInconclusive };
+// kNoRoot where the four corners lie on one side of the ray.
+template <class T> __device__ __forceinline__ Reach reduce(const F3* corner, F3 dir, Planar<T>& f)
 {
-    bool retry = false;
-    out = Hits{};
     const P3<T> w = {T(dir.x), T(dir.y), T(dir.z)};
     unsigned kz = 0;
     if (absv(w.y) > absv(w.x)) kz = 1;
@@ -153,12 +162,11 @@ template <class T> __device__ bool solve(const F3* corner, F3 dir, Hits& out)
     const P3<T> eu = sub(p1, p0), ev = sub(p2, p0), tw = sub(sub(p3, p2), eu);
     P2<T> a = project(p0, w, kz), b = project(eu, w, kz), c = project(ev, w, kz), d = project(tw, w, kz);
     const T scale = maxv(maxv(big(a), big(b)), maxv(big(c), big(d)));
-    if (!(scale > T(0))) return true;
+    if (!(scale > T(0))) return kInconclusive;
     a = mul(a, T(1) / scale);
     b = mul(b, T(1) / scale);
     c = mul(c, T(1) / scale);
     d = mul(d, T(1) / scale);
-    const T eps = Num<T>::eps;
     const P2<T> cs[4] = {a, add(a, b), add(a, c), add(add(add(a, b), c), d)};
     T xlo = cs[0].x, xhi = xlo, ylo = cs[0].y, yhi = ylo;
     for (unsigned i = 1; i < 4; ++i) {
@@ -167,8 +175,21 @@ template <class T> __device__ bool solve(const F3* corner, F3 dir, Hits& out)
         ylo = ylo < cs[i].y ? ylo : cs[i].y;
         yhi = maxv(yhi, cs[i].y);
     }
-    const T guard = T(64) * eps;
-    if (xlo > guard || xhi < -guard || ylo > guard || yhi < -guard) return false;
+    f = {w, p0, p1, p2, p3, a, b, c, d, kz};
+    const T guard = T(64) * Num<T>::eps;
+    return xlo > guard || xhi < -guard || ylo > guard || yhi < -guard ? kNoRoot : kMaybeRoot;
+}
+template <class T> __device__ __forceinline__ bool solve(const F3* corner, F3 dir, Hits& out)
+{
+    bool retry = false;
+    out = Hits{};
+    Planar<T> f;
+    const Reach reach = reduce<T>(corner, dir, f);
+    if (reach != kMaybeRoot) return reach == kInconclusive;
+    const P3<T> w = f.w, p0 = f.p0, p1 = f.p1, p2 = f.p2, p3 = f.p3;
+    const P2<T> a = f.a, b = f.b, c = f.c, d = f.d;
+    const unsigned kz = f.kz;
+    const T eps = Num<T>::eps, guard = T(64) * eps;
     const T A = crs(b, d), B = crs(a, d) + crs(b, c), Cc = crs(a, c);
     const T mag = maxv(absv(A), maxv(absv(B), absv(Cc)));
     if (!(mag > T(0))) return true;
@@ -201,6 +222,7 @@ template <class T> __device__ bool solve(const F3* corner, F3 dir, Hits& out)
             nroot = 2;
         }
     }
+#pragma unroll 1
     for (unsigned r = 0; r < nroot; ++r) {
         T u = roots[r];
         if (!(u == u)) { retry = true; continue; }
@@ -211,6 +233,7 @@ template <class T> __device__ bool solve(const F3* corner, F3 dir, Hits& out)
         if (!(v == v)) { retry = true; continue; }
         if (v < -guard || v > T(1) + guard) continue;
         T cond = T(1);
+#pragma unroll 1
         for (unsigned it = 0; it < 3; ++it) {
             const P2<T> fu = add(b, mul(d, v)), fv = add(c, mul(d, u));
             const T det = crs(fu, fv);
@@ -257,29 +280,34 @@ template <class T> __device__ bool solve(const F3* corner, F3 dir, Hits& out)
     return retry;
 }
 
-__device__ Hits intersect(const F3* c, F3 dir)
+__device__ __forceinline__ bool corners_ok(const F3* c)
 {
-    Hits r{};
-    const float n2 = fdot(dir, dir);
-    if (!(finite32(dir.x) && finite32(dir.y) && finite32(dir.z)) || !(n2 > 0.99f && n2 < 1.01f)) {
-        r.flags = bInvalid;
-        return r;
-    }
     for (unsigned i = 0; i < 4; ++i)
-        if (!(finite32(c[i].x) && finite32(c[i].y) && finite32(c[i].z)) || !(fdot(c[i], c[i]) <= 4.0f)) {
-            r.flags = bInvalid;
-            return r;
-        }
-    if (solve<float>(c, dir, r)) {
-        const bool unresolved = solve<double>(c, dir, r);
-        r.flags |= bFp64;
-        if (unresolved) r.flags |= bUnresolved;
-    }
+        if (!(finite32(c[i].x) && finite32(c[i].y) && finite32(c[i].z)) || !(fdot(c[i], c[i]) <= 4.0f)) return false;
+    return true;
+}
+__device__ __forceinline__ void order_roots(Hits& r)
+{
     if (r.count == 2 && (r.hit[1].u < r.hit[0].u || (r.hit[1].u == r.hit[0].u && r.hit[1].v < r.hit[0].v))) {
         const Hit t = r.hit[0];
         r.hit[0] = r.hit[1];
         r.hit[1] = t;
     }
+}
+__device__ Hits intersect(const F3* c, F3 dir)
+{
+    Hits r{};
+    const float n2 = fdot(dir, dir);
+    if (!(finite32(dir.x) && finite32(dir.y) && finite32(dir.z)) || !(n2 > 0.99f && n2 < 1.01f) || !corners_ok(c)) {
+        r.flags = bInvalid;
+        return r;
+    }
+    if (solve<float>(c, dir, r)) {
+        const bool unresolved = solve<double>(c, dir, r);
+        r.flags |= bFp64;
+        if (unresolved) r.flags |= bUnresolved;
+    }
+    order_roots(r);
     return r;
 }
 
@@ -300,6 +328,25 @@ __device__ __forceinline__ bool ray_box(F3 dir, const icp_patch_aabb& b)
     }
     return tnear <= tfar;
 }
+// False only where ray_box is false: the six divisions replaced by products with the direction's
+// rounded reciprocals (0 for an axis that is left out), each within 2^-22 of its quotient; the margins
+// are four times that.  Same comparisons, so that non-finite boxes fall the same way; infinite distances
+// fail the last comparison and are left to ray_box.
+__device__ __forceinline__ bool ray_box_maybe(F3 inv, const icp_patch_aabb& b)
+{
+    const float lo[3] = {b.min_x, b.min_y, b.min_z}, hi[3] = {b.max_x, b.max_y, b.max_z}, r[3] = {inv.x, inv.y, inv.z};
+    float tnear = 0.0f, tfar = 4.0f;
+#pragma unroll
+    for (unsigned a = 0; a < 3; ++a) {
+        const float t1 = lo[a] * r[a], t2 = hi[a] * r[a];
+        const bool use = r[a] != 0.0f;
+        const float tmin = t1 < t2 ? t1 : t2, tmax = t1 < t2 ? t2 : t1;
+        if (use && tmin > tnear) tnear = tmin;
+        if (use && tmax < tfar) tfar = tmax;
+    }
+    return !(tnear > tfar + ((tnear + fabsf(tfar)) * 0x1p-20f + 0x1p-120f));
+}
+__device__ __forceinline__ float box_reciprocal(float d) { return fabsf(d) > 0x1p-100f ? 1.0f / d : 0.0f; }
 
 // ------------------------------------------------------------------ direction bins
 __device__ __forceinline__ int bin_row(double z)
@@ -352,8 +399,8 @@ __device__ CapBins cap_bins(const icp_patch_aabb& b)
     const double tc = acos(fmin(1.0, fmax(-1.0, c[2])));
     const double dt = kPi / kBinRows, dp = 2 * kPi / kBinCols;
     CapBins out;
-    out.r0 = int(floor((tc - r) / dt)) - 1;
-    out.r1 = int(floor((tc + r) / dt)) + 1;
+    out.r0 = int(floor((tc - r) / dt));
+    out.r1 = int(floor((tc + r) / dt));
     if (tc - r <= 0 || tc + r >= kPi) { // the cap holds a pole
         out.r0 = out.r0 < 0 ? 0 : out.r0;
         out.r1 = out.r1 >= kBinRows ? kBinRows - 1 : out.r1;
@@ -370,7 +417,7 @@ __device__ CapBins cap_bins(const icp_patch_aabb& b)
         return out;
     }
     const double half = asin(s), pc = atan2(c[1], c[0]);
-    const int c0 = int(floor((pc - half + kPi) / dp)) - 1, c1 = int(floor((pc + half + kPi) / dp)) + 1;
+    const int c0 = int(floor((pc - half + kPi) / dp)), c1 = int(floor((pc + half + kPi) / dp));
     out.nc = c1 - c0 + 1;
     if (out.nc >= kBinCols) {
         out.c0 = 0;
@@ -499,59 +546,70 @@ struct RootCache {
     uint32_t* first;
 };
 
-// The same for a warp's 32 directions together.  Each lane runs the box test over its own bin list
-// and queues the few boxes its ray meets; the solver then takes 32 queued (direction, patch) pairs at a
-// time, so that it runs with a full warp (lane by lane 7 of 32 lanes were active: 2.33 -> 1.39 ms for
-// the 513 x 513 lattice at 360 x 720 directions).  The order in which a
-// direction's roots are found does not matter (the fill sorts them, and the noted flags and first
-// problem patch are order-independent).
-constexpr unsigned kPairQueue = 64; // a step adds at most 32 to at most 31 left over
+// The same for a warp's 32 directions together.  Each lane runs the box test over its own bin list; what
+// passes goes through three queues of (patch, lane) pairs, and each stage takes 32 pairs at a time, so that
+// it runs with a full warp whatever its share of the pairs is: the exact box test and the corners' side
+// (a quarter of the pairs go on), the binary32 solution, the binary64 solution (every second direction has
+// one).  One copy of each stage in one loop: the pass waits for instructions more than for memory.
+// The order in which a direction's roots are found does not matter (the fill sorts them, and the noted
+// flags and first problem patch are order-independent).
 struct PairQueue {
-    uint32_t patch[kPairQueue];
-    uint8_t lane[kPairQueue];
+    uint32_t patch[64]; // a push adds at most 32 to at most 31 left over
+    uint8_t lane[64];
 };
+// All lanes; n is warp-uniform.
+__device__ __forceinline__ void push(PairQueue& q, unsigned& n, bool want, uint32_t patch, uint32_t lane)
+{
+    const unsigned vote = __ballot_sync(0xffffffffu, want);
+    if (want) {
+        const unsigned at = n + __popc(vote & ((1u << (threadIdx.x & 31u)) - 1u));
+        q.patch[at] = patch;
+        q.lane[at] = (uint8_t)lane;
+    }
+    n += __popc(vote);
+    __syncwarp();
+}
+// The last (up to) 32 pairs; false for a lane that gets none.
+__device__ __forceinline__ bool pop(const PairQueue& q, unsigned& n, uint32_t& patch, uint32_t& lane)
+{
+    const unsigned me = threadIdx.x & 31u, m = n < 32u ? n : 32u;
+    n -= m;
+    if (me < m) {
+        patch = q.patch[n + me];
+        lane = q.lane[n + me];
+    }
+    __syncwarp();
+    return me < m;
+}
 struct WarpCollect {
-    PairQueue queue;
+    PairQueue near, side, refine;
     uint32_t count[32], flags[32], first[32];
     F3 dir[32];
 };
-
-__device__ void solve_pairs(const QueryArgs& q, WarpCollect& W, unsigned n, uint32_t first_direction, icp_query_hit* cached)
+__device__ __forceinline__ bool load_corners(const QueryArgs& q, const icp_outgoing_patch& p, F3* c)
 {
-    const unsigned lane = threadIdx.x & 31u;
-    if (lane < n) {
-        const uint32_t k = W.queue.patch[lane], d = W.queue.lane[lane];
-        const icp_outgoing_patch& p = q.patches[k];
-        F3 c[4];
-        bool bad = false;
-        for (unsigned j = 0; j < 4; ++j) {
-            if (p.vertex_indices[j] >= q.vertex_count) {
-                bad = true;
-                break;
-            }
-            c[j] = f3(q.vertices[p.vertex_indices[j]].direction_drop);
-        }
-        if (bad) {
-            atomicOr(&W.flags[d], (uint32_t)qInvalid);
-        } else {
-            const Hits h = intersect(c, W.dir[d]);
-            uint32_t flags = 0;
-            if (h.flags & (bUnresolved | bInvalid)) atomicMin(&W.first[d], p.patch_id);
-            if (h.flags & bUnresolved) flags |= qUnresolved;
-            if (h.flags & bInvalid) flags |= qInvalid;
-            if (h.flags & bFp64) flags |= qFp64;
-            for (uint32_t r = 0; r < h.count; ++r) {
-                const uint32_t at = atomicAdd(&W.count[d], 1u);
-                if (!cached) continue;
-                if (at >= kCachedRoots) flags |= qMismatch;
-                else
-                    cached[(size_t)(first_direction + d) * kCachedRoots + at] = {
-                        k, p.patch_id, r, h.hit[r].flags, h.hit[r].u, h.hit[r].v, h.hit[r].t, h.hit[r].residual};
-            }
-            if (flags) atomicOr(&W.flags[d], flags);
-        }
+    for (unsigned j = 0; j < 4; ++j) {
+        if (p.vertex_indices[j] >= q.vertex_count) return false;
+        c[j] = f3(q.vertices[p.vertex_indices[j]].direction_drop);
     }
-    __syncwarp();
+    return true;
+}
+__device__ __forceinline__ void note(const QueryArgs& q, WarpCollect& W, uint32_t k, uint32_t d, const Hits& h,
+                                     icp_query_hit* cached)
+{
+    const uint32_t id = q.patches[k].patch_id;
+    uint32_t flags = 0;
+    if (h.flags & (bUnresolved | bInvalid)) atomicMin(&W.first[d], id);
+    if (h.flags & bUnresolved) flags |= qUnresolved;
+    if (h.flags & bInvalid) flags |= qInvalid;
+    if (h.flags & bFp64) flags |= qFp64;
+    for (uint32_t r = 0; r < h.count; ++r) {
+        const uint32_t at = atomicAdd(&W.count[d], 1u);
+        if (!cached) continue;
+        if (at >= kCachedRoots) flags |= qMismatch;
+        else cached[(size_t)d * kCachedRoots + at] = {k, id, r, h.hit[r].flags, h.hit[r].u, h.hit[r].v, h.hit[r].t, h.hit[r].residual};
+    }
+    if (flags) atomicOr(&W.flags[d], flags);
 }
 
 __global__ void __launch_bounds__(kThreads, kQueryBlocksPerSm) query_count_kernel(QueryArgs q, unsigned long long* __restrict__ counts,
@@ -559,7 +617,7 @@ __global__ void __launch_bounds__(kThreads, kQueryBlocksPerSm) query_count_kerne
 {
     __shared__ WarpCollect warps[kThreads / 32];
     WarpCollect& W = warps[threadIdx.x >> 5];
-    const unsigned lane = threadIdx.x & 31u, before = (1u << lane) - 1u;
+    const unsigned lane = threadIdx.x & 31u;
     for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < q.direction_count;
          base += gridDim.x * blockDim.x) {
         const uint32_t i = base + lane;
@@ -579,43 +637,66 @@ __global__ void __launch_bounds__(kThreads, kQueryBlocksPerSm) query_count_kerne
             }
         }
         W.dir[lane] = dir;
+        const F3 inv = {box_reciprocal(dir.x), box_reciprocal(dir.y), box_reciprocal(dir.z)};
+        icp_query_hit* const cached = cache.hits ? cache.hits + (size_t)base * kCachedRoots : nullptr;
         __syncwarp();
-        unsigned queued = 0;
-        while (__any_sync(0xffffffffu, s < end)) {
-            uint32_t k = 0;
-            bool met = false;
-            if (s < end) {
-                k = q.bin_list[s++];
-                met = ray_box(dir, q.boxes[k]);
+        unsigned near = 0, side = 0, refine = 0; // pairs queued
+        for (;;) {
+            const bool more = __any_sync(0xffffffffu, s < end);
+            uint32_t k = 0, d = lane;
+            if (more) {
+                bool want = false;
+                if (s < end) {
+                    k = q.bin_list[s++];
+                    want = ray_box_maybe(inv, q.boxes[k]);
+                }
+                push(W.near, near, want, k, lane);
             }
-            const unsigned vote = __ballot_sync(0xffffffffu, met);
-            if (!vote) continue;
-            if (met) {
-                const unsigned at = queued + __popc(vote & before);
-                W.queue.patch[at] = k;
-                W.queue.lane[at] = (uint8_t)lane;
-            }
-            queued += __popc(vote);
-            __syncwarp();
-            if (queued >= 32u) {
-                solve_pairs(q, W, 32u, base, cache.hits);
-                // the rest moves to the front
-                queued -= 32u;
-                uint32_t mp = 0;
-                uint8_t ml = 0;
-                if (lane < queued) {
-                    mp = W.queue.patch[32u + lane];
-                    ml = W.queue.lane[32u + lane];
+            if (near >= 32u || (!more && near)) {
+                Reach reach = kNoRoot;
+                if (pop(W.near, near, k, d) && ray_box(W.dir[d], q.boxes[k])) {
+                    F3 c[4];
+                    Planar<float> f;
+                    if (!load_corners(q, q.patches[k], c)) atomicOr(&W.flags[d], (uint32_t)qInvalid);
+                    else if (!corners_ok(c)) {
+                        Hits bad{};
+                        bad.flags = bInvalid;
+                        note(q, W, k, d, bad, nullptr);
+                    } else
+                        reach = reduce<float>(c, W.dir[d], f);
                 }
                 __syncwarp();
-                if (lane < queued) {
-                    W.queue.patch[lane] = mp;
-                    W.queue.lane[lane] = ml;
+                push(W.side, side, reach != kNoRoot, k, d);
+            }
+            if (side >= 32u || (!more && !near && side)) {
+                bool retry = false;
+                if (pop(W.side, side, k, d)) {
+                    F3 c[4];
+                    Hits h;
+                    load_corners(q, q.patches[k], c);
+                    retry = solve<float>(c, W.dir[d], h);
+                    if (!retry) {
+                        order_roots(h);
+                        note(q, W, k, d, h, cached);
+                    }
+                }
+                __syncwarp();
+                push(W.refine, refine, retry, k, d);
+            }
+            if (refine >= 32u || (!more && !near && !side && refine)) {
+                if (pop(W.refine, refine, k, d)) {
+                    F3 c[4];
+                    Hits h;
+                    load_corners(q, q.patches[k], c);
+                    const bool unresolved = solve<double>(c, W.dir[d], h);
+                    h.flags |= unresolved ? bFp64 | bUnresolved : bFp64;
+                    order_roots(h);
+                    note(q, W, k, d, h, cached);
                 }
                 __syncwarp();
             }
+            if (!more && !near && !side && !refine) break;
         }
-        if (queued) solve_pairs(q, W, queued, base, cache.hits);
         if (i < q.direction_count) {
             counts[i] = W.count[lane];
             if (cache.hits) {
