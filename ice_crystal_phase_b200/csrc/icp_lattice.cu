@@ -88,21 +88,22 @@ template <class T> __host__ __device__ __forceinline__ T root(T x)
     else return sqrt(x);
 }
 // nextUp: the least representable number above x (+inf and NaN unchanged, either zero to the
-// least positive subnormal); nextDown(x) = -nextUp(-x).
-// Adding +0 turns -0 into +0, whose successor is then the general one.
-__device__ __forceinline__ float next_up(float x)
-{
-    const int b = __float_as_int(x + 0.0f);
-    return x < INFINITY ? __int_as_float(b + ((b >> 31) | 1)) : x;
-}
-__device__ __forceinline__ double next_up(double x)
-{
-    const long long b = __double_as_longlong(x + 0.0);
-    return x < (double)INFINITY ? __longlong_as_double(b + ((b >> 63) | 1ll)) : x;
-}
-template <class T> __device__ __forceinline__ T next_down(T x) { return -next_up(-x); }
+// least positive subnormal); nextDown(x) = -nextUp(-x).  x plus the least subnormal, rounded up, is
+// that number for every x but -inf (checked over all 2^32 binary32 values): one addition where the
+// step on the bits took six operations, and an enclosure is made of little else.  An enclosure
+// whose finite end has overflowed stays infinite, on the side that excludes it already.
+__device__ __forceinline__ float next_up(float x) { return __fadd_ru(x, 0x1p-149f); }
+__device__ __forceinline__ double next_up(double x) { return __dadd_ru(x, 0x1p-1074); }
+__device__ __forceinline__ float next_down(float x) { return __fadd_rd(x, -0x1p-149f); }
+__device__ __forceinline__ double next_down(double x) { return __dadd_rd(x, -0x1p-1074); }
 template <class T> __device__ __forceinline__ T lesser(T a, T b) { return a < b ? a : b; }
 template <class T> __device__ __forceinline__ T greater(T a, T b) { return a > b ? a : b; }
+// The same for products that are stepped outward next (which leaves no sign to a zero) and are NaN
+// all together or not at all: one instruction each.
+__device__ __forceinline__ float least(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ double least(double a, double b) { return lesser(a, b); }
+__device__ __forceinline__ float most(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double most(double a, double b) { return greater(a, b); }
 template <class T> __device__ __forceinline__ T magnitude(T x) { return x < T(0) ? -x : x; }
 template <class T> __device__ __forceinline__ T infinity_of() { return T(INFINITY); }
 
@@ -152,17 +153,17 @@ template <class T> __device__ __forceinline__ Iv<T> operator-(Iv<T> a, Iv<T> b) 
 template <class T> __device__ __forceinline__ Iv<T> operator*(Iv<T> a, Iv<T> b)
 {
     const T p = a.lo * b.lo, q = a.lo * b.hi, r = a.hi * b.lo, s = a.hi * b.hi;
-    return {next_down(lesser(lesser(p, q), lesser(r, s))), next_up(greater(greater(p, q), greater(r, s)))};
+    return {next_down(least(least(p, q), least(r, s))), next_up(most(most(p, q), most(r, s)))};
 }
-template <class T> __device__ __forceinline__ Iv<T> operator/(Iv<T> a, Iv<T> b)
+// 1 / a for a.lo > 0
+template <class T> __device__ __forceinline__ Iv<T> reciprocal(Iv<T> a)
 {
-    if (b.lo <= T(0) && b.hi >= T(0)) return {-infinity_of<T>(), infinity_of<T>()};
-    return a * Iv<T>{next_down(T(1) / b.hi), next_up(T(1) / b.lo)};
+    return {next_down(T(1) / a.hi), next_up(T(1) / a.lo)};
 }
 template <class T> __device__ __forceinline__ Iv<T> squared(Iv<T> a)
 {
     const T p = a.lo * a.lo, q = a.hi * a.hi;
-    return {a.lo <= T(0) && a.hi >= T(0) ? T(0) : greater(T(0), next_down(lesser(p, q))), next_up(greater(p, q))};
+    return {a.lo <= T(0) && a.hi >= T(0) ? T(0) : greater(T(0), next_down(least(p, q))), next_up(most(p, q))};
 }
 template <class T> __device__ __forceinline__ Iv<T> square_root(Iv<T> a)
 {
@@ -215,6 +216,19 @@ template <class T> __device__ __forceinline__ V<T> gradient(const Shape& S, V<T>
     return u - (V<T>{T(0), T(-1), T(0)} - u * mu) * (derivative / r);
 }
 
+// implicit at p and the slope of it along w (the gradient's product with w), from one length and one
+// series.
+template <class T> __device__ __forceinline__ T implicit_and_slope(const Shape& S, V<T> p, V<T> w, T& slope)
+{
+    const T r = length(p);
+    const V<T> u = p / r;
+    T derivative;
+    const T mu = -u.y;
+    const T radius = series(S, mu, derivative);
+    slope = dot(u - (V<T>{T(0), T(-1), T(0)} - u * mu) * (derivative / r), w);
+    return r < T(S.inner) * T(0.25) ? r - T(S.inner) : r - radius;
+}
+
 template <class T> struct Bounds {
     Iv<T> value, derivative;
 };
@@ -231,13 +245,15 @@ template <class T> __device__ __forceinline__ Bounds<T> bound_surface(const Shap
     if (r.hi < T(S.inner)) return {{-T(1), -T(1)}, {-inf, inf}};
     if (r.lo > T(S.outer)) return {{T(1), T(1)}, {-inf, inf}};
     if (r.lo <= T(0)) return {{-inf, inf}, {-inf, inf}};
-    I mu = (-py) / r;
+    const I per_r = reciprocal(r);
+    I mu = (-py) * per_r;
     mu.lo = greater(mu.lo, -T(1));
     mu.hi = lesser(mu.hi, T(1));
     I previous = at_point(T(1)), current = mu, dp = at_point(T(0)), dc = at_point(T(1));
     I radius = at_point(T(1)) + at_point(T(S.c[0])) + at_point(T(S.c[1])) * mu;
     I slope = at_point(T(S.c[1]));
     const I two = at_point(T(2));
+#pragma unroll 1 // unrolled: 5 % slower, instructions again
     for (unsigned n = 2; n <= S.last; ++n) {
         const I next = two * mu * current - previous;
         const I dn = two * current + two * mu * dc - dp;
@@ -250,15 +266,9 @@ template <class T> __device__ __forceinline__ Bounds<T> bound_surface(const Shap
         dp = dc;
         dc = dn;
     }
-    const I dr = (px * at_point(w.x) + py * at_point(w.y) + pz * at_point(w.z)) / r;
-    const I dm = (at_point(-w.y) - mu * dr) / r;
+    const I dr = (px * at_point(w.x) + py * at_point(w.y) + pz * at_point(w.z)) * per_r;
+    const I dm = (at_point(-w.y) - mu * dr) * per_r;
     return {r - radius, dr - slope * dm};
-}
-
-// The same out of line: the end checks of a monotone bracket, and the binary64 retry.
-template <class T> __device__ __noinline__ Bounds<T> bound_surface_call(const Shape& S, V<T> o, V<T> w, T lower, T upper)
-{
-    return bound_surface(S, o, w, lower, upper);
 }
 
 struct Query {
@@ -284,57 +294,79 @@ template <class T> __device__ __forceinline__ Root<T> solve_surface(const Shape&
         const T f = implicit(S, along(o, w, start));
         if (!(f < T(0))) return {kCodeUnresolved, T(0)}; // a grazing chord is not skipped silently
     }
-    Segment<T> stack[64];
+    // One enclosure a step, whichever one the lane needs next: of a segment, or of either end of a
+    // monotone one.  A bracket leaves the loop and is refined after it (one exit, so that the lanes of
+    // a warp meet there and refine theirs together).
+    Segment<T> stack[64], s{start, limit};
     unsigned size = 0, visits = 0;
-    stack[size++] = {start, limit};
-    while (size != 0) {
-        if (++visits > 16384u) return {kCodeUnresolved, T(0)};
-        const Segment<T> s = stack[--size];
-        Bounds<T> b;
-        if constexpr (std::is_same_v<T, float>) b = bound_surface(S, o, w, s.lo, s.hi);
-        else b = bound_surface_call(S, o, w, s.lo, s.hi);
-        if (excludes_zero(b.value)) continue;
-        const T mid = s.lo + (s.hi - s.lo) * T(0.5);
-        const T width_tolerance = tolerance * greater(T(1), magnitude(mid));
-        if (excludes_zero(b.derivative)) {
-            T lo = s.lo, hi = s.hi;
-            T f_lo = implicit(S, along(o, w, lo));
-            T f_hi = implicit(S, along(o, w, hi));
-            if ((f_lo < T(0)) == (f_hi < T(0))) {
-                // monotone with equal end signs: excluded once the end values' signs are certain
-                const Iv<T> left = bound_surface_call(S, o, w, lo, lo).value;
-                const Iv<T> right = bound_surface_call(S, o, w, hi, hi).value;
-                if ((left.lo > T(0) && right.lo > T(0)) || (left.hi < T(0) && right.hi < T(0))) continue;
-            }
-            if (f_lo == T(0) && lo > start) return {kCodeHit, lo};
-            if (f_hi == T(0) && hi > start) return {kCodeHit, hi};
-            if ((f_lo < T(0)) != (f_hi < T(0))) {
-                T x = mid;
-                for (unsigned it = 0; it < 96u; ++it) {
-                    const V<T> p = along(o, w, x);
-                    const T f = implicit(S, p);
-                    if (f == T(0) || hi - lo <= width_tolerance) return {kCodeHit, x};
-                    if ((f < T(0)) == (f_lo < T(0))) {
-                        lo = x;
-                        f_lo = f;
-                    } else {
-                        hi = x;
-                        f_hi = f;
-                    }
-                    const T slope = dot(gradient(S, p), w);
-                    const T candidate = x - f / slope;
-                    const T guard = (hi - lo) * T(0.1);
-                    x = candidate > lo + guard && candidate < hi - guard ? candidate : lo + (hi - lo) * T(0.5);
-                }
-                return {kCodeUnresolved, T(0)};
-            }
+    stack[size++] = s;
+    enum { kSegment, kLeft, kRight } step = kSegment;
+    bool left_above = false;
+    T f_lo = T(0), f_hi = T(0);
+    bool bracket = false;
+    Root<T> found{kCodeUnresolved, T(0)};
+    for (;;) {
+        if (step == kSegment) {
+            if (size == 0) found.code = kCodeMiss;
+            if (size == 0 || ++visits > 16384u) break;
+            s = stack[--size];
         }
-        if (s.hi - s.lo <= width_tolerance || mid == s.lo || mid == s.hi || size + 2 > 64u)
-            return {kCodeUnresolved, T(0)};
+        const Bounds<T> b = bound_surface(S, o, w, step == kRight ? s.hi : s.lo, step == kLeft ? s.lo : s.hi);
+        if (step == kSegment) {
+            if (excludes_zero(b.value)) continue;
+            if (excludes_zero(b.derivative)) {
+                f_lo = implicit(S, along(o, w, s.lo));
+                f_hi = implicit(S, along(o, w, s.hi));
+                if ((f_lo < T(0)) == (f_hi < T(0))) {
+                    // monotone with equal end signs: excluded once the end values' signs are certain
+                    step = kLeft;
+                    continue;
+                }
+                if (f_lo == T(0) && s.lo > start) found = {kCodeHit, s.lo};
+                else if (f_hi == T(0) && s.hi > start) found = {kCodeHit, s.hi};
+                else bracket = true;
+                break;
+            }
+        } else {
+            const bool certain = excludes_zero(b.value), above = b.value.lo > T(0);
+            if (step == kLeft && certain) {
+                left_above = above;
+                step = kRight;
+                continue;
+            }
+            const bool excluded = step == kRight && certain && above == left_above;
+            step = kSegment;
+            if (excluded) continue;
+            if (f_lo == T(0) && s.lo > start) found = {kCodeHit, s.lo};
+            else if (f_hi == T(0) && s.hi > start) found = {kCodeHit, s.hi};
+            if (found.code == kCodeHit) break;
+        }
+        const T mid = s.lo + (s.hi - s.lo) * T(0.5);
+        if (s.hi - s.lo <= tolerance * greater(T(1), magnitude(mid)) || mid == s.lo || mid == s.hi || size + 2 > 64u) break;
         stack[size++] = {mid, s.hi};
         stack[size++] = {s.lo, mid};
     }
-    return {kCodeMiss, T(0)};
+    if (bracket) {
+        T lo = s.lo, hi = s.hi, x = lo + (hi - lo) * T(0.5);
+        const T width_tolerance = tolerance * greater(T(1), magnitude(x));
+        for (unsigned it = 0; it < 96u; ++it) {
+            T slope;
+            const T f = implicit_and_slope(S, along(o, w, x), w, slope);
+            if (f == T(0) || hi - lo <= width_tolerance) {
+                found = {kCodeHit, x};
+                break;
+            }
+            if ((f < T(0)) == (f_lo < T(0))) {
+                lo = x;
+                f_lo = f;
+            } else
+                hi = x;
+            const T candidate = x - f / slope;
+            const T guard = (hi - lo) * T(0.1);
+            x = candidate > lo + guard && candidate < hi - guard ? candidate : lo + (hi - lo) * T(0.5);
+        }
+    }
+    return found;
 }
 
 // The binary64 retry on its own: rare, and its code stays out of the way of the binary32 loop.
@@ -351,9 +383,11 @@ __device__ Hit intersect(const Shape& S, const Query& q)
     Hit h{kCodeMiss, {0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}, 0u};
     const Root<float> r = solve_surface<float>(S, q);
     bool fallback = r.code == kCodeUnresolved;
+    F3 point{0.0f, 0.0f, 0.0f}, normal{0.0f, 0.0f, 0.0f};
     if (r.code == kCodeHit) {
-        const F3 p = along(q.origin, q.direction, r.distance);
-        const float incidence = fabsf(dot(unit(gradient(S, p)), q.direction));
+        point = along(q.origin, q.direction, r.distance);
+        normal = unit(gradient(S, point));
+        const float incidence = fabsf(dot(normal, q.direction));
         fallback = incidence < 0.05f; // grazing: binary32 is ill-conditioned there
     }
     h.code = r.code;
@@ -367,8 +401,8 @@ __device__ Hit intersect(const Shape& S, const Query& q)
             h.normal = unit(to<float>(unit(gradient(S, p))));
         }
     } else if (r.code == kCodeHit) {
-        h.position = along(q.origin, q.direction, r.distance);
-        h.normal = unit(gradient(S, h.position));
+        h.position = point;
+        h.normal = normal;
     }
     return h;
 }
@@ -597,12 +631,13 @@ struct BlockTally {
     unsigned long long first_problem;
 };
 
-// What bounds it: instruction supply and the dependent chains of the interval enclosures (15 % of the
-// issue slots; no memory traffic to speak of).  With the solver inlined for the entry and again for
-// the internal encounters, each with three enclosures and a binary64 copy, half of a warp's time
-// went into waiting for instructions: 6.3 ms at 513 x 513.  One copy in one loop, the rare parts out
-// of line: 2.2 ms.  (80 registers and six blocks per SM: 2.5 ms, the enclosure out of line: 2.4 ms.)
-__global__ void __launch_bounds__(kThreads) lattice_trace_kernel(const __grid_constant__ TraceArgs A,
+// What bounds it: instruction supply and the dependent chains of the interval enclosures (a quarter of
+// the issue slots; no memory traffic to speak of), with half of the lanes waiting for the warp's longest
+// search.  Figures for 513 x 513 rays, 6.3 ms with the solver inlined for the entry and again for the
+// internal encounters: one copy of it in one loop 2.2 ms, outward steps of one instruction 1.3 ms, one
+// enclosure a step and one exit before the refinement 0.91 ms.  Four blocks per SM (128 registers, a few
+// spills) are as good as five and 5 % better than three; one place that writes the records was no faster.
+__global__ void __launch_bounds__(kThreads, 4) lattice_trace_kernel(const __grid_constant__ TraceArgs A,
                                                                  icp_outgoing_vertex* __restrict__ vertices,
                                                                  icp_field32* __restrict__ second,
                                                                  unsigned long long* __restrict__ tally)

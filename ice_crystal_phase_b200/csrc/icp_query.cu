@@ -57,9 +57,9 @@ int ok()
     } while (0)
 
 constexpr unsigned kThreads = 128;
-// The counting pass waits on candidate gathers and on instructions; six blocks per SM (80 registers,
-// a few bytes of spills) do as well as four or eight (within 0.5 % of each other).
-constexpr unsigned kQueryBlocksPerSm = 6;
+// Four blocks per SM leave the counting pass 128 registers and no spills; six at 80 registers spill and
+// cost 0.1 ms more at 513 x 513 and 360 x 720 directions.
+constexpr unsigned kQueryBlocksPerSm = 4;
 constexpr unsigned kScanThreads = 1024;
 constexpr int kBinRows = 256, kBinCols = 512;
 constexpr double kPi = 3.141592653589793238462643383279502884;
