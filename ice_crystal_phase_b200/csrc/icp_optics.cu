@@ -494,38 +494,55 @@ struct Panel {
     double u0, u1, z0, z1;
     unsigned depth;
 };
-// Tensor Gauss rule over a panel of the branch: u across [u0, u1], v = the section's
-// [lo, hi] mapped from z in [z0, z1].
-__device__ Integral fold_quadrature(const Fold& g, int sign, const Panel& p, bool high)
+constexpr unsigned kFoldLow = 8, kFoldHigh = 16, kFoldPoints = kFoldLow * kFoldLow + kFoldHigh * kFoldHigh;
+struct FoldTerms {
+    double of[4][kFoldPoints + 1]; // area, mu, mv, omega; the 8 x 8 points, then the 16 x 16 ones
+};
+// Tensor Gauss rules of both orders over a panel of the branch: u across [u0, u1], v = the section's
+// [lo, hi] mapped from z in [z0, z1].  The whole warp calls it with the same arguments: the lanes
+// evaluate the points, ten each, and eight lanes add up one sum each in the order of the points (u outer),
+// as a loop over them would; points outside the section add nothing.
+__device__ void fold_quadrature(const Fold& g, int sign, const Panel& p, FoldTerms& terms, Integral& low, Integral& high)
 {
-    const unsigned n = high ? 16u : 8u;
+    const unsigned lane = threadIdx.x & 31u;
     const double uh = (p.u1 - p.u0) * 0.5, uc = (p.u0 + p.u1) * 0.5;
     const double zh = (p.z1 - p.z0) * 0.5, zc = (p.z0 + p.z1) * 0.5;
-    Integral s{0, 0, 0, 0};
-    for (unsigned i = 0; i < n; ++i) {
-        double xi, wi;
-        gl_point(high, i, xi, wi);
+    for (unsigned e = lane; e < kFoldPoints; e += 32u) {
+        const bool order16 = e >= kFoldLow * kFoldLow;
+        const unsigned at = order16 ? e - kFoldLow * kFoldLow : e, n = order16 ? kFoldHigh : kFoldLow;
+        double xi, wi, xk, wk;
+        gl_point(order16, at / n, xi, wi);
+        gl_point(order16, at % n, xk, wk);
         const double u = fma(uh, xi, uc);
-        double vl = 0, vh = 0;
-        if (!fold_section(g.j, sign, u, vl, vh)) continue;
-        const double width = vh - vl;
-        for (unsigned k = 0; k < n; ++k) {
-            double xk, wk;
-            gl_point(high, k, xk, wk);
+        double vl = 0, vh = 0, w = 0, wu = 0, wv = 0, wj = 0;
+        if (fold_section(g.j, sign, u, vl, vh)) {
+            const double width = vh - vl;
             const double z = fma(zh, xk, zc), v = fma(z, width, vl);
-            const double w = uh * zh * wi * wk * width;
+            w = uh * zh * wi * wk * width;
             const D3 pt = fold_point(g, u, v);
             const double q = dot(pt, pt);
             const double J = fabs(bilinear4(g.j, u, v)) * g.scale;
-            s.area += w;
-            s.mu += w * u;
-            s.mv += w * v;
-            s.omega += w * J / (q * sqrt(q));
+            wu = w * u;
+            wv = w * v;
+            wj = w * J / (q * sqrt(q));
         }
+        terms.of[0][e] = w;
+        terms.of[1][e] = wu;
+        terms.of[2][e] = wv;
+        terms.of[3][e] = wj;
     }
-    return s;
+    __syncwarp();
+    double sum = 0;
+    const unsigned begin = lane < 4u ? kFoldLow * kFoldLow : 0u, end = lane < 4u ? kFoldPoints : lane < 8u ? kFoldLow * kFoldLow : 0u;
+#pragma unroll 8
+    for (unsigned e = begin; e < end; ++e) sum += terms.of[lane & 3u][e];
+    __syncwarp(); // the terms are read before the next panel's are written
+    const unsigned all = 0xffffffffu;
+    high = {__shfl_sync(all, sum, 0), __shfl_sync(all, sum, 1), __shfl_sync(all, sum, 2), __shfl_sync(all, sum, 3)};
+    low = {__shfl_sync(all, sum, 4), __shfl_sync(all, sum, 5), __shfl_sync(all, sum, 6), __shfl_sync(all, sum, 7)};
 }
-__device__ bool fold_integrate(const Fold& g, icp_folded_branch& b, const icp_folded_config& c, icp_folded_record& r)
+__device__ bool fold_integrate(const Fold& g, icp_folded_branch& b, const icp_folded_config& c, icp_folded_record& r,
+                               FoldTerms& terms)
 {
     double cuts[4] = {0, 0, 0, 0};
     const unsigned n = fold_cuts(g, cuts);
@@ -541,7 +558,8 @@ __device__ bool fold_integrate(const Fold& g, icp_folded_branch& b, const icp_fo
         while (size) {
             const Panel p = stack[--size];
             if (++r.panels > c.maximum_panels) return false;
-            const Integral low = fold_quadrature(g, b.sign, p, false), high = fold_quadrature(g, b.sign, p, true);
+            Integral low, high;
+            fold_quadrature(g, b.sign, p, terms, low, high);
             if (!(high.area > 0 && high.omega > 0 && finite64(high.area) && finite64(high.omega))) return false;
             const double ea = fabs(high.area - low.area) / high.area;
             const double es = fabs(high.omega - low.omega) / high.omega;
@@ -596,10 +614,12 @@ __device__ __forceinline__ void fold_blank(icp_folded_record& r, uint32_t patch_
     r.flags = kFoldInvalidInput;
     for (unsigned i = 0; i < 4; ++i) r.branches[i].focal_flags = kFocalInputPending;
 }
-// FoldedPatchBuilder::prepare: the record of one NeedsRefinement patch (status 3).
+// FoldedPatchBuilder::prepare: the record of one NeedsRefinement patch (status 3).  A warp prepares a patch:
+// every lane runs all of it on the same values but for the quadrature's points.
 __device__ void fold_prepare(const icp_outgoing_vertex* __restrict__ vertices, uint32_t vertex_count,
                              const icp_outgoing_patch& patch, uint32_t compact, F3 incident,
-                             const icp_focal_config* focal, const icp_folded_config& config, icp_folded_record& r)
+                             const icp_focal_config* focal, const icp_folded_config& config, icp_folded_record& r,
+                             FoldTerms& terms)
 {
     fold_blank(r, patch.patch_id, compact);
     if (!vertices || patch.status != 3u || !(patch.incident_area_drop2 > 0) ||
@@ -628,7 +648,7 @@ __device__ void fold_prepare(const icp_outgoing_vertex* __restrict__ vertices, u
     }
     double area = 0;
     for (unsigned i = 0; i < r.branch_count; ++i) {
-        if (!fold_integrate(g, r.branches[i], config, r)) {
+        if (!fold_integrate(g, r.branches[i], config, r, terms)) {
             r.flags = kFoldUnconverged;
             return;
         }
@@ -953,7 +973,9 @@ __device__ void direction_optics(const icp_optics_input& in, uint32_t index, con
     }
 }
 
-__global__ void __launch_bounds__(kThreads) patch_optics_kernel(const icp_optics_input in, const icp_focal_config fc,
+// Waits on gathers of patches, vertices and hits: four blocks per SM at 128 registers (0.41 ms for 360 x 720
+// directions of the 513 x 513 lattice) where the two that 230 registers leave took 0.53 ms; five: the same.
+__global__ void __launch_bounds__(kThreads, 4) patch_optics_kernel(const icp_optics_input in, const icp_focal_config fc,
                                                                 int with_focal, const FoldView folded,
                                                                 icp_optical_result* __restrict__ results,
                                                                 icp_focal_sample* __restrict__ focal)
@@ -1041,18 +1063,25 @@ __global__ void __launch_bounds__(kFoldThreads) fold_slot_kernel(const icp_outgo
 // one thread per record: the quadrature's panel count varies, so the records are dense and
 // the launch covers only them.  acc: [0] prepared, [1] unresolved, [2] branches, [3] focal-
 // pending branches, [4] largest estimated error (bits of a non-negative double)
-__global__ void __launch_bounds__(64) fold_prepare_kernel(const icp_outgoing_vertex* __restrict__ vertices,
+// A thousand candidates or so lie along the caustics of a 513 x 513 lattice: one thread each kept 18
+// blocks busy for 0.39 ms, a serial chain of some thousand quadrature points with a root and two quotients
+// in each.  A warp each: 0.05 ms.
+constexpr unsigned kFoldWarps = 2;
+__global__ void __launch_bounds__(kFoldWarps * 32) fold_prepare_kernel(const icp_outgoing_vertex* __restrict__ vertices,
                                                           uint32_t vertex_count, const icp_outgoing_patch* __restrict__ patches,
                                                           const uint32_t* __restrict__ list, uint32_t count, F3 incident,
                                                           icp_focal_config focal, int with_focal, icp_folded_config config,
                                                           icp_folded_record* __restrict__ records,
                                                           unsigned long long* __restrict__ acc)
 {
-    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ FoldTerms terms[kFoldWarps];
+    const uint32_t slot = blockIdx.x * kFoldWarps + threadIdx.x / 32u;
     if (slot >= count) return;
     const uint32_t compact = list[slot];
     icp_folded_record r;
-    fold_prepare(vertices, vertex_count, patches[compact], compact, incident, with_focal ? &focal : nullptr, config, r);
+    fold_prepare(vertices, vertex_count, patches[compact], compact, incident, with_focal ? &focal : nullptr, config, r,
+                 terms[threadIdx.x / 32u]);
+    if (threadIdx.x & 31u) return;
     records[slot] = r;
     if (r.flags == kFoldReady) {
         atomicAdd(&acc[0], 1ull);
@@ -1233,7 +1262,7 @@ extern "C" int icp_folded_prepare(icp_context* ctx, const icp_outgoing_vertex* d
         return fail(ICP_ERR_CAPACITY, "icp_folded_prepare: %u folded-patch records need room, capacity is %u", n, capacity);
     ICP_CUDA(cudaMemsetAsync(acc, 0, 5 * sizeof(unsigned long long), ctx->stream));
     const icp_focal_config fc = focal ? *focal : icp_focal_config{};
-    fold_prepare_kernel<<<(n + 63) / 64, 64, 0, ctx->stream>>>(d_vertices, vertex_count, d_patches, list, n,
+    fold_prepare_kernel<<<(n + kFoldWarps - 1) / kFoldWarps, kFoldWarps * 32, 0, ctx->stream>>>(d_vertices, vertex_count, d_patches, list, n,
                                                                F3{incident[0], incident[1], incident[2]}, fc,
                                                                focal ? 1 : 0, cfg, d_records, acc);
     ICP_CUDA(cudaGetLastError());
