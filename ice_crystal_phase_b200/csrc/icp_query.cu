@@ -383,18 +383,18 @@ __device__ CapBins cap_bins(const icp_patch_aabb& b)
         const double p[3] = {(k & 1) ? hi[0] : lo[0], (k & 2) ? hi[1] : lo[1], (k & 4) ? hi[2] : lo[2]};
         const double n = sqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
         if (!(n > 0)) return all;
+        const double per_n = 1.0 / n;
         for (unsigned a = 0; a < 3; ++a) {
-            dirs[k][a] = p[a] / n;
+            dirs[k][a] = p[a] * per_n;
             c[a] += dirs[k][a];
         }
     }
     const double cn = sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
     if (!(cn > 0)) return all;
     for (unsigned a = 0; a < 3; ++a) c[a] /= cn;
-    double r = 0;
-    for (unsigned k = 0; k < 8; ++k)
-        r = fmax(r, acos(fmin(1.0, fmax(-1.0, c[0] * dirs[k][0] + c[1] * dirs[k][1] + c[2] * dirs[k][2]))));
-    r += kCapMargin;
+    double widest = 1.0; // the cosine of the corner farthest from the axis
+    for (unsigned k = 0; k < 8; ++k) widest = fmin(widest, c[0] * dirs[k][0] + c[1] * dirs[k][1] + c[2] * dirs[k][2]);
+    const double r = acos(fmax(-1.0, widest)) + kCapMargin;
     if (!(r < 0.5 * kPi)) return all; // larger than a hemisphere: not convex, take everything
     const double tc = acos(fmin(1.0, fmax(-1.0, c[2])));
     const double dt = kPi / kBinRows, dp = 2 * kPi / kBinCols;
@@ -430,7 +430,7 @@ __device__ CapBins cap_bins(const icp_patch_aabb& b)
 // f(bin, patch) for every bin of every patch's cap.  A thread walks its own cap when that is small;
 // the caps of a pole or of a box around the origin cover up to all 131072 bins, and a warp walks each
 // of those together: one thread alone waits for a returning atomic per bin (fill 0.65 -> 0.27 ms for
-// the 513 x 513 lattice).
+// the 513 x 513 lattice; with caps that take no spare bins and one arc cosine for a cap's width 0.14 ms).
 constexpr int kWideCap = 64; // bins
 template <class F> __device__ __forceinline__ void for_cap_bins(const icp_patch_aabb* boxes, uint32_t patch_count, F f)
 {
@@ -550,7 +550,8 @@ struct RootCache {
 // passes goes through three queues of (patch, lane) pairs, and each stage takes 32 pairs at a time, so that
 // it runs with a full warp whatever its share of the pairs is: the exact box test and the corners' side
 // (a quarter of the pairs go on), the binary32 solution, the binary64 solution (every second direction has
-// one).  One copy of each stage in one loop: the pass waits for instructions more than for memory.
+// one).  One copy of each stage in one loop.  Lane by lane 7 of 32 lanes were active: 2.33 -> 0.60 ms for the
+// 513 x 513 lattice at 360 x 720 directions.
 // The order in which a direction's roots are found does not matter (the fill sorts them, and the noted
 // flags and first problem patch are order-independent).
 struct PairQueue {
