@@ -110,11 +110,11 @@ __device__ __forceinline__ uint64_t rng_bits(uint64_t seed, uint64_t id, unsigne
 }
 // Midpoints of 2^52 cells (the reference's draw, exact in binary64).
 __device__ __forceinline__ double uniform_f64(uint64_t bits) { return (double(bits >> 12) + 0.5) * 0x1p-52; }
-// FP32 path: the same 64-bit draw rounded to float (round-to-nearest of the 52-bit midpoint,
-// kept strictly below 1).
+// FP32 path: the same 64-bit draw rounded to float (round-to-nearest of the 52-bit midpoint, one
+// conversion of the odd 53-bit integer, kept strictly below 1).
 __device__ __forceinline__ float uniform_f32(uint64_t bits)
 {
-    const float u = __double2float_rn(uniform_f64(bits));
+    const float u = __ull2float_rn((bits >> 12) * 2u + 1u) * 0x1p-53f;
     return u < 1.0f ? u : 0.99999994f;
 }
 template <class R> __device__ __forceinline__ R uniform(uint64_t bits);
