@@ -87,12 +87,20 @@ struct AtlasTrace {
     unsigned long long* cells; // nt*np
     unsigned long long* acc;   // [0] forward pole, [1] backward pole, [2] exits outside the grid
     AtlasAudit* audits;
+    uint32_t warp_rays; // rays per warp, 1..32
 };
 
-__global__ void __launch_bounds__(128) atlas_trace_kernel(const AtlasTrace P)
+// A node waits for its longest ray, a serial chain of encounters, and has a few hundred rays: they are
+// spread over the chip's warps, one ray or a few in each, so that an encounter runs the code of its own
+// kind only (most of a long chain is total reflection, which bins nothing).  With 32 rays to a warp every
+// encounter ran every kind.
+constexpr unsigned kAtlasWarps = 4;   // per block
+constexpr unsigned kAtlasSpread = 8;  // warps per SM before a warp takes more rays
+__global__ void __launch_bounds__(kAtlasWarps * 32) atlas_trace_kernel(const AtlasTrace P)
 {
-    const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= P.count) return;
+    const unsigned lane = threadIdx.x & 31u;
+    const uint64_t id = ((uint64_t)blockIdx.x * kAtlasWarps + threadIdx.x / 32u) * P.warp_rays + lane;
+    if (lane >= P.warp_rays || id >= P.count) return;
     const icp_atlas_ray q = P.rays[id];
     const double wscale = q.weight_mm2 * P.scale;
     double esc = 0, esc_c = 0;
@@ -620,7 +628,10 @@ int icp_atlas_trace_node(icp_context* ctx, const icp_atlas_settings* s, uint32_t
         ICP_CUDA(cudaMemcpyAsync(d_rays, rays.data() + first, n * sizeof(icp_atlas_ray), cudaMemcpyHostToDevice,
                                  stream));
         P.count = n;
-        atlas_trace_kernel<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(P);
+        P.warp_rays = 1;
+        while (P.warp_rays < 32u && n > uint64_t(ctx->sms) * kAtlasSpread * P.warp_rays) P.warp_rays *= 2u;
+        const uint64_t per_block = uint64_t(kAtlasWarps) * P.warp_rays;
+        atlas_trace_kernel<<<(unsigned)((n + per_block - 1) / per_block), kAtlasWarps * 32, 0, stream>>>(P);
         ICP_CUDA(cudaGetLastError());
         count_launch();
         ICP_CUDA(cudaMemcpyAsync(audits.data(), d_audit, n * sizeof(AtlasAudit), cudaMemcpyDeviceToHost, stream));
