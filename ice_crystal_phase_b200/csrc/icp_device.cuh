@@ -231,43 +231,42 @@ __device__ __forceinline__ Interface<R> split(V3<R> d, V3<R> e, Stokes<R> S, V3<
 // |d x n| scaled by its largest component so that the refraction cosine, and the exit direction,
 // round identically).  What the two kinds of reflection share -- a square root, two reciprocals, two
 // quotients -- is evaluated once with selected operands; only the phase of a total reflection
-// is left to a branch.
-__device__ __forceinline__ Interface<double> split(V3<double> d, V3<double> e, Stokes<double> S, V3<double> n,
-                                                   const Media<double>& M)
+// is left to a branch.  In pieces, by what they depend on: the directions (incidence, reflected), the
+// frame (fresnel), the polarisation (pass).
+struct Incidence {
+    V3<double> s; // s-polarisation unit vector, meaningless where sine is 0
+    double sine, ci;
+};
+__device__ __forceinline__ double incidence_cosine(V3<double> d, V3<double> n) { return rmin(1.0, rmax(0.0, -dot(d, n))); }
+__device__ __forceinline__ Incidence incidence(V3<double> d, V3<double> n)
 {
-    Interface<double> out;
-    if (M.matched) {
-        out.s = e;
-        out.dt = d;
-        out.t = S;
-        out.dr = unit(d - n * (2.0 * dot(d, n)));
-        out.r = {0.0, 0.0, 0.0, 0.0};
-        out.ci = -dot(d, n);
-        out.has_t = true;
-        out.tir = false;
-        out.balance = 0.0;
-        return out;
-    }
-    double ci = -dot(d, n);
-    ci = rmin(1.0, rmax(0.0, ci));
-    V3<double> s = cross(d, n);
+    const V3<double> s = cross(d, n);
     const double scale = fmax(fabs(s.x), fmax(fabs(s.y), fabs(s.z)));
     const V3<double> t = quot(s, div_by(scale));
     const double len = sqrt(dot(t, t));
-    const double sine = scale > 0 ? scale * len : 0.0;
-    s = quot(t, div_by(len));
-    if (!(sine > 0)) s = e;
-    out.s = s;
-    // Basis rotation (e, d x e) -> (s, d x s): c = e.s, sg = (d x e).s
+    return {quot(t, div_by(len)), scale > 0 ? scale * len : 0.0, incidence_cosine(d, n)};
+}
+__device__ __forceinline__ V3<double> reflected(V3<double> d, V3<double> n, const Media<double>& M)
+{
+    if (M.matched) return unit(d - n * (2.0 * dot(d, n)));
+    return unit(d + n * (2.0 * incidence_cosine(d, n)));
+}
+struct Fresnel {
+    double cos2, sin2p; // basis rotation (e, d x e) -> (s, d x s)
+    double Rs, Rp, zr, zi;
+    V3<double> dt;
+    bool tir;
+};
+__device__ __forceinline__ Fresnel fresnel(V3<double> d, V3<double> e, V3<double> n, V3<double> s, double sine, double ci,
+                                           const Media<double>& M)
+{
+    Fresnel F;
     const double c = dot(e, s);
     const double sg = dot(cross(d, e), s);
-    const double cos2 = c * c - sg * sg, sin2p = 2.0 * c * sg;
-    const double Q = cos2 * S.Q + sin2p * S.U;
-    const double U = -sin2p * S.Q + cos2 * S.U;
+    F.cos2 = c * c - sg * sg;
+    F.sin2p = 2.0 * c * sg;
     const double a = M.a, b = M.b;
     const double st = M.eta * sine;
-    out.dr = unit(d + n * (2.0 * ci));
-    out.ci = ci;
     const bool tir = st > 1.0;
     const double inv = __drcp_rn(tir ? st : 2.0);
     const double root = sqrt(tir ? (1.0 - inv) * (1.0 + inv) : (1.0 - st) * (1.0 + st));
@@ -276,44 +275,75 @@ __device__ __forceinline__ Interface<double> split(V3<double> d, V3<double> e, S
     const DivBy D1 = div_by(tir ? rmax(rabs(aci), rabs(bu)) : aci + bu);
     const DivBy D2 = div_by(tir ? rmax(rabs(bci), rabs(au)) : bci + au);
     const double q1 = quot(tir ? aci : aci - bu, D1), q2 = quot(tir ? bci : bci - au, D2);
-    double Rs, Rp, zr, zi;
     if (tir) {
         const double x1 = q1, x2 = q2, y1 = quot(bu, D1), y2 = quot(au, D2);
         const DivBy E1 = div_by(x1 * x1 + y1 * y1), E2 = div_by(x2 * x2 + y2 * y2);
         const double rsr = quot(x1 * x1 - y1 * y1, E1), rsi = quot(-2.0 * x1 * y1, E1);
         const double rpr = quot(x2 * x2 - y2 * y2, E2), rpi = quot(-2.0 * x2 * y2, E2);
-        Rs = 1.0;
-        Rp = 1.0;
-        zr = rsr * rpr + rsi * rpi; // rs * conj(rp)
-        zi = rsi * rpr - rsr * rpi;
+        F.Rs = 1.0;
+        F.Rp = 1.0;
+        F.zr = rsr * rpr + rsi * rpi; // rs * conj(rp)
+        F.zi = rsi * rpr - rsr * rpi;
+        F.dt = d;
     } else {
-        Rs = q1 * q1;
-        Rp = q2 * q2;
-        zr = q1 * q2;
-        zi = 0.0;
+        F.Rs = q1 * q1;
+        F.Rp = q2 * q2;
+        F.zr = q1 * q2;
+        F.zi = 0.0;
+        F.dt = unit((d + n * ci) * M.eta - n * root);
     }
-    out.tir = tir;
-    out.has_t = !tir;
-    const double hs = 0.5 * (Rs + Rp), hd = 0.5 * (Rs - Rp);
-    out.r.I = hs * S.I + hd * Q;
-    out.r.Q = hd * S.I + hs * Q;
-    out.r.U = zr * U - zi * S.V;
-    out.r.V = zi * U + zr * S.V;
-    double lost;
-    if (!tir) {
-        out.dt = unit((d + n * ci) * M.eta - n * root);
-        const double zt = sqrt((1.0 - Rs) * (1.0 - Rp));
+    F.tir = tir;
+    return F;
+}
+// The reflected Stokes vector; Q and U of the incident one in the new frame.
+__device__ __forceinline__ Stokes<double> pass(const Fresnel& F, Stokes<double> S, double& Q, double& U)
+{
+    Q = F.cos2 * S.Q + F.sin2p * S.U;
+    U = -F.sin2p * S.Q + F.cos2 * S.U;
+    const double hs = 0.5 * (F.Rs + F.Rp), hd = 0.5 * (F.Rs - F.Rp);
+    return {hs * S.I + hd * Q, hd * S.I + hs * Q, F.zr * U - F.zi * S.V, F.zi * U + F.zr * S.V};
+}
+// Relative power imbalance of a split of power I into r and (unless totally reflected) t.
+__device__ __forceinline__ double imbalance(double I, double r, double t, bool tir)
+{
+    const double lost = tir ? rabs(r - I) : rabs(r + t - I);
+    return I > 0.0 ? quot(lost, div_by(I)) : 0.0;
+}
+__device__ __forceinline__ Interface<double> split(V3<double> d, V3<double> e, Stokes<double> S, V3<double> n,
+                                                   const Media<double>& M)
+{
+    Interface<double> out;
+    out.dr = reflected(d, n, M);
+    if (M.matched) {
+        out.s = e;
+        out.dt = d;
+        out.t = S;
+        out.r = {0.0, 0.0, 0.0, 0.0};
+        out.ci = -dot(d, n);
+        out.has_t = true;
+        out.tir = false;
+        out.balance = 0.0;
+        return out;
+    }
+    const Incidence in = incidence(d, n);
+    out.s = in.sine > 0 ? in.s : e;
+    out.ci = in.ci;
+    const Fresnel F = fresnel(d, e, n, out.s, in.sine, in.ci, M);
+    double Q, U;
+    out.r = pass(F, S, Q, U);
+    out.tir = F.tir;
+    out.has_t = !F.tir;
+    out.dt = F.dt;
+    if (!F.tir) {
+        const double zt = sqrt((1.0 - F.Rs) * (1.0 - F.Rp));
         out.t.I = S.I - out.r.I;
         out.t.Q = Q - out.r.Q;
         out.t.U = zt * U;
         out.t.V = zt * S.V;
-        lost = rabs(out.r.I + out.t.I - S.I);
     } else {
-        out.dt = d;
         out.t = {0.0, 0.0, 0.0, 0.0};
-        lost = rabs(out.r.I - S.I);
     }
-    out.balance = S.I > 0.0 ? quot(lost, div_by(S.I)) : 0.0;
+    out.balance = imbalance(S.I, out.r.I, out.t.I, F.tir);
     return out;
 }
 
