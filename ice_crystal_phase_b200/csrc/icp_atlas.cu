@@ -247,25 +247,31 @@ __global__ void __launch_bounds__(32) atlas_chain_kernel(const AtlasTrace P)
         bool stopped = status >= 0;
         for (uint32_t enc = 0; !stopped && enc < P.max_hits;) {
             // where the ray goes
-            V3<double> md{0, 0, 1}, mn{0, 0, -1};
+            V3<double> md{0, 0, 1}, mp{0, 0, 0};
+            double best = 0, second = 0;
+            unsigned mface = 0;
             int mstatus = 0;
             unsigned count = 0;
 #pragma unroll 1
             while (count < kChain && enc + count < P.max_hits) {
-                double t;
-                const Boundary hit = next_boundary(P.geo, p, d, face, t);
-                const V3<double> n = -face_normal<double>(hit.face);
+                double t1, t2;
+                const Boundary hit = nearest_plane(P.geo, p, d, face, t1, t2);
                 if (lane == count) {
                     md = d;
-                    mn = n;
+                    mp = p;
+                    mface = hit.face;
                     mstatus = hit.status;
+                    best = t1;
+                    second = t2;
                 }
                 ++count;
                 if (hit.status) break;
-                d = reflected(d, n, P.leave);
+                d = reflected(d, -face_normal<double>(hit.face), P.leave);
                 face = hit.face;
             }
             // the encounters side by side
+            if (lane < count && mstatus == 0) mstatus = boundary_status(P.geo, mp, mface, best, second);
+            const V3<double> mn = -face_normal<double>(mface);
             Incidence in = incidence(md, mn);
             unsigned kept = __ballot_sync(kFull, lane < count && (P.leave.matched || !(in.sine > 0)));
             while (kept) { // no plane of incidence: the frame before stays

@@ -203,14 +203,17 @@ __device__ __forceinline__ double rcp_rough(double x)
 // runner-up is within the rough quotients' error does every candidate get its exact distance (the
 // reference's tie rule needs both).  The point itself was checked against `start` when it
 // was reached (strict_face_point below and at the entry), so it is not checked again here.
-__device__ __forceinline__ Boundary next_boundary(const HexGeo<double>& P, V3<double>& p, V3<double> d, unsigned start,
-                                                  double& t_out)
+// In two parts: the plane and the point on it (nearest_plane; status 5 without one), and whether they are
+// certain (boundary_status).
+__device__ __forceinline__ Boundary nearest_plane(const HexGeo<double>& P, V3<double>& p, V3<double> d, unsigned start,
+                                                  double& best, double& second)
 {
     Boundary out{8u, 0, false};
     const Axes<double> D = prism_axes(d), A = prism_axes(p);
     if (axis_of(D, start) > 128 * Eps<double>::eps) { out.status = 5; return out; }
     const double none = 1.7976931348623157e308;
-    double best = none, second = none, gap = 0, slope = 1;
+    best = second = none;
+    double gap = 0, slope = 1;
     double num[4];
     bool valid[4];
 #pragma unroll
@@ -252,9 +255,19 @@ __device__ __forceinline__ Boundary next_boundary(const HexGeo<double>& P, V3<do
         second = none; // further than the tolerance below
     }
     p = p + d * best;
-    t_out = best;
+    return out;
+}
+__device__ __forceinline__ int boundary_status(const HexGeo<double>& P, V3<double> p, unsigned face, double best, double second)
+{
     const double tol = 128 * Eps<double>::eps * fmax(1.0, fmax(P.half_len, fmax(fmax(fabs(p.x), fmax(fabs(p.y), fabs(p.z))), fabs(best))));
-    if (second - best <= tol || !strict_face_point(P, p, out.face)) out.status = 3;
+    return second - best <= tol || !strict_face_point(P, p, face) ? 3 : 0;
+}
+__device__ __forceinline__ Boundary next_boundary(const HexGeo<double>& P, V3<double>& p, V3<double> d, unsigned start,
+                                                  double& t_out)
+{
+    double second;
+    Boundary out = nearest_plane(P, p, d, start, t_out, second);
+    if (!out.status) out.status = boundary_status(P, p, out.face, t_out, second);
     return out;
 }
 
