@@ -160,6 +160,65 @@ __device__ __forceinline__ void pack_bf16(const float (&v)[2][32], uint32_t (&w)
         }
 }
 
+// The same for 32 columns: 64-byte rows in 2 KB, the four chunks of row r exchanged by r / 2 mod 4.
+constexpr uint32_t kHalfTileBytes = kTileBytes / 2u;
+__device__ __forceinline__ uint4* half_chunk(uint8_t* buf, uint32_t row, uint32_t ch)
+{
+    return reinterpret_cast<uint4*>(buf + row * 64u + ((ch ^ ((row >> 1) & 3u)) << 4));
+}
+__device__ __forceinline__ void load_half_tile(const __nv_bfloat16* src, uint32_t ld, uint32_t lane, uint4 (&part)[4])
+{
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i)
+        part[i] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(8u * i + (lane >> 2)) * ld + 8u * (lane & 3u)));
+}
+
+// Columns [c0, c1) (a multiple of 32) of a warp's 32 rows through the backward epilogue: the activation's
+// derivative at z_prev, the BF16 store and the bias gradient.  Half the width of epilogue_layer's step, so
+// that sixteen warps fit: what bounds it is the latency of its chain (tensor memory, two special functions,
+// 31 shuffles, two passes through shared memory).  z holds the first 32 columns of z_prev.
+template <int N>
+__device__ __forceinline__ void epilogue_backprop(const GemmArgs& g, uint32_t taddr, uint32_t m0, uint32_t lane,
+                                                  uint32_t c0, uint32_t c1, float* colsum, uint4 (&z)[4], uint8_t* buf)
+{
+#pragma unroll 1
+    for (uint32_t c = c0; c < c1; c += 32u) {
+        float v[32];
+        umma::tmem_ld32(taddr + c, v);
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) *half_chunk(buf, 8u * i + (lane >> 2), lane & 3u) = z[i];
+        if (c + 32u < c1) load_half_tile(g.z_prev + (size_t)m0 * N + c + 32u, N, lane, z);
+        __syncwarp();
+        // this lane's row: chunk by chunk, in place
+#pragma unroll
+        for (uint32_t ch = 0; ch < 4; ++ch) {
+            uint4* const at = half_chunk(buf, lane, ch);
+            const uint4 u = *at;
+            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+            uint32_t o[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float* x = &v[8 * ch + 2 * i];
+                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+                x[0] *= silu_grad<false>(f.x);
+                x[1] *= silu_grad<false>(f.y);
+                const __nv_bfloat162 p = __floats2bfloat162_rn(x[0], x[1]);
+                o[i] = *reinterpret_cast<const uint32_t*>(&p);
+            }
+            *at = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+        __syncwarp();
+        __nv_bfloat16* const dst = g.out_dz + (size_t)m0 * N + c;
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            const uint32_t row = 8u * i + (lane >> 2), ch = lane & 3u;
+            *reinterpret_cast<uint4*>(dst + (size_t)row * N + 8u * ch) = *half_chunk(buf, row, ch);
+        }
+        __syncwarp();
+        atomicAdd(&colsum[c + lane], warp_column_sum(v, lane));
+    }
+}
+
 // Columns [0, N) of one row of a 128 x N accumulator tile to FP32 (kStoreF32, kAtomicF32): this
 // thread's TMEM lane starts at taddr, m is the output row.
 template <int EPI>
@@ -380,21 +439,24 @@ __global__ void __launch_bounds__(128, 1)
 // the whole B (N x K BF16, <= 128 KB) stays in shared memory; one CTA per SM walks the 128-row
 // tiles t = blockIdx.x, blockIdx.x + gridDim.x, ...  Warp 0 streams A chunks through a deep ring
 // with TMA; warp 1 allocates 2 N TMEM columns and one of its threads issues the MMAs into
-// accumulator buffer (tile & 1); the kEpiWarps warps 2.. drain the other buffer through the
+// accumulator buffer (tile & 1); the epilogue warps 2.. drain the other buffer through the
 // fused epilogue, so a tile's epilogue overlaps the next tile's MMAs.  Epilogue warp w reads
 // TMEM lanes 32 (w mod 4) .. (the rows its lane quarter may access) and column slice
-// (w - 2) / 4 of kEpiWarps / 4; the head's partial sums of a row meet in shared memory behind
+// (w - 2) / 4; the head's partial sums of a row meet in shared memory behind
 // a named barrier per lane quarter.  Bias and head weights are staged in shared memory.
 // Barriers: a_full / a_empty per ring stage, b_full, acc_full / acc_empty per accumulator, and
 // drain (all MMAs complete).  Every wait is bounded; a role that gives up raises the abort flag
 // and the error word, the others give up at their next wait, in-flight loads and MMAs are
 // waited for, and the tensor memory is freed.
-constexpr uint32_t kEpiWarps = 8;
-constexpr uint32_t kSlices = kEpiWarps / 4;
-constexpr uint32_t kPThreads = 64 + 32 * kEpiWarps;
-// per-CTA extras after the ring: barriers (1 KB), colsum, bias, head weights (1 KB each), head
-// partial sums (kSlices - 1 slices x 128 floats, rounded up to kSlices)
-constexpr int kPExtra = 1024 + 3 * 1024 + (int)kSlices * 512 + (int)(kEpiWarps * kTileBytes);
+// Sixteen warps in the backward epilogue, which reads, transforms, sums and stores (0.91 ms with eight for
+// 16 records of 131072 rows, the reads and stores alone 0.50), eight in the others.
+template <int EPI> __host__ __device__ constexpr uint32_t epi_warps() { return EPI == kBackprop ? 16u : 8u; }
+template <int EPI> __host__ __device__ constexpr uint32_t epi_slices() { return epi_warps<EPI>() / 4u; }
+template <int EPI> __host__ __device__ constexpr uint32_t epi_threads() { return 64u + 32u * epi_warps<EPI>(); }
+// per-CTA extras after the ring: barriers (1 KB), colsum, bias, head weights (1 KB each), the head's
+// partial sums (of its second slice, rounded up), the tile buffers
+constexpr int kPExtra = 1024 + 3 * 1024 + 2 * 512 + (int)(8u * kTileBytes);
+static_assert(16u * kHalfTileBytes == 8u * kTileBytes, "tile buffers");
 template <int N, int KC> __host__ __device__ constexpr int pstages()
 {
     return (232448 - 1024 - N * 128 * KC - kPExtra) / (int)kA > 8 ? 8
@@ -411,16 +473,17 @@ __device__ __forceinline__ void named_sync(uint32_t id, uint32_t threads)
 }
 
 template <int N, int KC, int EPI>
-__global__ void __launch_bounds__(kPThreads, 1)
+__global__ void __launch_bounds__(epi_threads<EPI>(), 1)
     gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                            const GemmArgs g)
 {
     constexpr int S = pstages<N, KC>();
     constexpr bool kHeadEpi = EPI == kHead || EPI == kHeadTrain;
+    constexpr uint32_t kEpiWarps = epi_warps<EPI>(), kSlices = epi_slices<EPI>();
     constexpr uint32_t BB = (uint32_t)N * 128u;   // one 64-wide K chunk of B
     constexpr uint32_t W = (uint32_t)N / kSlices; // columns per epilogue warp
     static_assert(S >= 2, "ring too shallow");
-    static_assert(W % 64u == 0, "slice width: the epilogue takes columns in pairs of 32");
+    static_assert(W % (EPI == kBackprop ? 32u : 64u) == 0, "slice width: whole steps of the epilogue");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* bres = smem;
@@ -437,7 +500,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
     float* sbias = colsum + 256;
     float* shead = sbias + 256;
     float* ypart = shead + 256; // [kSlices - 1][128]
-    uint8_t* tbufs = reinterpret_cast<uint8_t*>(ypart + kSlices * 128u); // per epilogue warp
+    uint8_t* tbufs = reinterpret_cast<uint8_t*>(ypart + 256u); // per epilogue warp
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t tiles = g.M / 128u;
 
@@ -542,14 +605,14 @@ __global__ void __launch_bounds__(kPThreads, 1)
         const uint32_t q = warp & 3u, slice = (warp - 2u) >> 2;
         const uint32_t c0 = slice * W;
         const uint32_t row = 32u * q + lane;
-        uint8_t* buf = tbufs + (warp - 2u) * kTileBytes;
+        uint8_t* buf = tbufs + (warp - 2u) * (EPI == kBackprop ? kHalfTileBytes : kTileBytes);
         uint32_t i = 0;
         bool live = true;
 #pragma unroll 1
         for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
             const uint32_t b = i & 1u;
-            uint4 z[8]; // requested before the accumulator is waited for
-            if constexpr (EPI == kBackprop) load_tile(g.z_prev + (size_t)(t * 128u + 32u * q) * N + c0, N, lane, z);
+            uint4 z[EPI == kBackprop ? 4 : 8]; // requested before the accumulator is waited for
+            if constexpr (EPI == kBackprop) load_half_tile(g.z_prev + (size_t)(t * 128u + 32u * q) * N + c0, N, lane, z);
             const bool mine = live && umma::mbar_wait(&acc_full[b], (i >> 1) & 1u, kWaitLimit);
             if (!__all_sync(0xffffffffu, mine && !*abort_flag)) {
                 if (lane == 0 && live) {
@@ -563,6 +626,8 @@ __global__ void __launch_bounds__(kPThreads, 1)
                 umma::fence_after_sync();
                 const uint32_t taddr = tmem + ((32u * q) << 16) + b * (uint32_t)N;
                 if constexpr (EPI == kStoreF32) epilogue_f32<EPI>(g, taddr, t * 128u + row, c0, c0 + W);
+                else if constexpr (EPI == kBackprop)
+                    epilogue_backprop<N>(g, taddr, t * 128u + 32u * q, lane, c0, c0 + W, colsum, z, buf);
                 else
                     y = epilogue_layer<N, EPI>(g, taddr, t * 128u + 32u * q, lane, c0, c0 + W, sbias, shead, colsum, z,
                                                buf);
@@ -680,7 +745,7 @@ template <int N, int KC, int EPI> int launch_p(const void* A, const void* B, con
     if (e != cudaSuccess) return (int)e;
     const uint32_t tiles = g.M / 128u;
     const uint32_t grid = tiles < (uint32_t)sm_count() ? tiles : (uint32_t)sm_count();
-    gemm_persistent_kernel<N, KC, EPI><<<grid, kPThreads, smem, st>>>(ta, tb, g);
+    gemm_persistent_kernel<N, KC, EPI><<<grid, epi_threads<EPI>(), smem, st>>>(ta, tb, g);
     return (int)cudaGetLastError();
 }
 
