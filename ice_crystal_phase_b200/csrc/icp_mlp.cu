@@ -24,16 +24,20 @@ __device__ __forceinline__ float silu_grad_of(float z)
     return s * (1.0f + z * (1.0f - s));
 }
 
-// X rows: thread per 8 BF16 (one uint4) of a row.
+// X rows: thread per 8 BF16 (one uint4) of a row.  A warp takes two neighbouring chunks of 16 rows (whole
+// 32-byte sectors), so that it copies record features, copies cell features or evaluates harmonics; a warp
+// of two rows ran all three, with half its lanes idle (0.26 ms for 16 records of 131072 rows; 0.15 ms so).
 __global__ void features_kernel(const uint4* __restrict__ rec16, const uint4* __restrict__ cells, uint32_t C,
-                                uint32_t q_row, uint32_t q_axis, uint64_t total, const double* __restrict__ recgeo,
+                                uint32_t q_row, uint32_t q_axis, uint32_t warps, const double* __restrict__ recgeo,
                                 const double* __restrict__ cellgeo, uint4* __restrict__ X)
 {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    const uint64_t m = t / q_row;
-    const uint32_t q = (uint32_t)(t - m * q_row);
-    const uint32_t r = (uint32_t)(m / C), c = (uint32_t)(m - (uint64_t)r * C);
+    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (w >= warps) return;
+    const uint32_t pairs = q_row / 2u, tile = w / pairs;
+    const uint32_t q = 2u * (w - tile * pairs) + (lane & 1u);
+    const uint32_t m = 16u * tile + (lane >> 1);
+    const uint32_t r = m / C, c = m - r * C;
+    const uint64_t t = (uint64_t)m * q_row + q;
     if (q < 2) {
         X[t] = rec16[2u * r + q];
     } else if (q < q_axis) {
@@ -245,11 +249,13 @@ int launch_features(const __nv_bfloat16* rec16, const __nv_bfloat16* cells, uint
 {
     if (K0 % 64 || C % 128 || !records || P % 8 || P + 16 > K0) return -1;
     const uint32_t q_row = K0 / 8u;
-    const uint64_t total = (uint64_t)records * C * q_row;
-    features_kernel<<<blocks_of(total, 256), 256, 0, st>>>(reinterpret_cast<const uint4*>(rec16),
-                                                           reinterpret_cast<const uint4*>(cells), C, q_row,
-                                                           q_row - P / 8u, total, recgeo, cellgeo,
-                                                           reinterpret_cast<uint4*>(X));
+    if ((uint64_t)records * C > 0xffffffffull) return -1;
+    const uint64_t warps = (uint64_t)records * C / 16u * (q_row / 2u); // C is a multiple of 128, q_row of 8
+    if (warps > 0xffffffffull) return -1;
+    features_kernel<<<blocks_of(warps * 32u, 256), 256, 0, st>>>(reinterpret_cast<const uint4*>(rec16),
+                                                                 reinterpret_cast<const uint4*>(cells), C, q_row,
+                                                                 q_row - P / 8u, (uint32_t)warps, recgeo, cellgeo,
+                                                                 reinterpret_cast<uint4*>(X));
     return (int)cudaGetLastError();
 }
 
