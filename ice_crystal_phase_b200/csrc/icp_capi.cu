@@ -580,7 +580,7 @@ namespace {
 // Strips per record of a batched build: 2, or the fewest of 4, 8, .. that fit shared memory (the
 // chains of a strip's columns run side by side, so wider strips cost little and let more records
 // share a launch).  per = records per co-resident launch; 0 when one launch per record is as good.
-// 32 records of 180 x 360 cells stored at 90 x 180: 0.96 ms one by one, 0.06 ms in one launch.
+// 32 records of 180 x 360 cells stored at 90 x 180: 0.96 ms one by one, 0.12 ms in one launch.
 icp_context::BatchShapeEntry cdf_batch_shape(icp_context* c, uint32_t nt, uint32_t np, uint32_t ct, uint32_t cp)
 {
     for (const auto& k : c->cdf_batch_shapes)
