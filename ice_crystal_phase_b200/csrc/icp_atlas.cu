@@ -185,7 +185,8 @@ __global__ void __launch_bounds__(kAtlasWarps * 32) atlas_trace_kernel(const Atl
 // encounters -- frame, Fresnel factors, refracted direction and its cell -- the lanes then do side by side,
 // and the power is a short recursion over their factors, in the old order.  Past the ray's end up to
 // kChain - 1 directions are made in vain.  28 nodes of 72 to 216 rays, with the host's part: 7.4 ms one thread
-// a ray and 32 to a warp, 6.0 ms one to a warp, 4.4 ms so (4.6 with 8 or 4.5 with 32 encounters at a time).
+// a ray and 32 to a warp, 6.0 ms one to a warp, 4.4 ms so (4.6 with 8 or 4.5 with 32 encounters at a time),
+// 4.0 ms with the certainty checks off the chain and one wait for the device a node.
 constexpr unsigned kChain = 16;
 // Rays per SM up to which each has a warp of its own: at 3456 rays (23 per SM) 28 nodes take 11.2 ms so and
 // 12.0 ms spread, at 7776 rays 21.7 and 17.9 ms.
@@ -788,6 +789,8 @@ int icp_atlas_trace_node(icp_context* ctx, const icp_atlas_settings* s, uint32_t
     report->projected_area_mm2 = area;
     report->rays = nr;
     std::vector<AtlasAudit> audits(chunk);
+    unsigned long long acc[4] = {};
+    const unsigned mblocks = (unsigned)std::min<uint64_t>((cells + 255) / 256, uint64_t(ctx->sms) * 8);
     AtlasAudit first_bad{};
     for (uint64_t first = 0; first < nr; first += chunk) {
         const uint64_t n = std::min(chunk, nr - first);
@@ -804,7 +807,14 @@ int icp_atlas_trace_node(icp_context* ctx, const icp_atlas_settings* s, uint32_t
         }
         ICP_CUDA(cudaGetLastError());
         count_launch();
+        if (first + n == nr) {
+            // the masses follow the last rays at once, so that the node waits for the device once
+            atlas_mass_kernel<<<mblocks, 256, 0, stream>>>(d_cells, d_acc, s->nt, s->np, total * kUnit62, d_mass, d_acc + 3);
+            ICP_CUDA(cudaGetLastError());
+            count_launch();
+        }
         ICP_CUDA(cudaMemcpyAsync(audits.data(), d_audit, n * sizeof(AtlasAudit), cudaMemcpyDeviceToHost, stream));
+        if (first + n == nr) ICP_CUDA(cudaMemcpyAsync(acc, d_acc, sizeof acc, cudaMemcpyDeviceToHost, stream));
         ICP_CUDA(cudaStreamSynchronize(stream));
         for (uint64_t q = 0; q < n; ++q) {
             const AtlasAudit& a = audits[q];
@@ -825,13 +835,6 @@ int icp_atlas_trace_node(icp_context* ctx, const icp_atlas_settings* s, uint32_t
             unresolved.add(rays[r].weight_mm2 * a.residual);
         }
     }
-    const unsigned mblocks = (unsigned)std::min<uint64_t>((cells + 255) / 256, uint64_t(ctx->sms) * 8);
-    atlas_mass_kernel<<<mblocks, 256, 0, stream>>>(d_cells, d_acc, s->nt, s->np, total * kUnit62, d_mass, d_acc + 3);
-    ICP_CUDA(cudaGetLastError());
-    count_launch();
-    unsigned long long acc[4];
-    ICP_CUDA(cudaMemcpyAsync(acc, d_acc, sizeof acc, cudaMemcpyDeviceToHost, stream));
-    ICP_CUDA(cudaStreamSynchronize(stream));
     report->invalid_bins = acc[2];
     report->escaped_mm2 = escaped.value;
     report->unresolved_mm2 = unresolved.value;
