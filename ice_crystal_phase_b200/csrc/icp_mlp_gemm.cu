@@ -26,6 +26,7 @@
 #include "icp_internal.h"
 #include "icp_mlp.h"
 #include "icp_mlp_features.cuh"
+#include "icp_packed.cuh"
 #include "icp_umma.cuh"
 
 namespace icp::mlp {
@@ -57,14 +58,6 @@ template <int N, int MT = 1> constexpr size_t smem_bytes()
 // y <- y (1 + e + e^2) (error cubed: 1.7e-8; 1.1e-7 after the binary32 roundings, measured over
 // a binade) -- five FMA-pipe operations.  z is clamped at -80 so that d stays finite; the
 // result then is below 2e-35.
-// 2^x on the special-function unit with subnormal results flushed (one instruction; the
-// exponential here is only ever added to 1).
-__device__ __forceinline__ float ex2_ftz(float x)
-{
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ float logistic(float z)
 {
     const float d = 1.0f + ex2_ftz(fmaxf(z, -80.0f) * -1.44269504088896341f);
@@ -200,8 +193,9 @@ __device__ __forceinline__ void epilogue_backprop(const GemmArgs& g, uint32_t ta
             for (int i = 0; i < 4; ++i) {
                 float* x = &v[8 * ch + 2 * i];
                 const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
-                x[0] *= silu_grad<false>(f.x);
-                x[1] *= silu_grad<false>(f.y);
+                uint64_t sg, grad;
+                silu_grad_pair(pk2(f.x, f.y), sg, grad);
+                upk2(mul2(pk2(x[0], x[1]), grad), x[0], x[1]);
                 const __nv_bfloat162 p = __floats2bfloat162_rn(x[0], x[1]);
                 o[i] = *reinterpret_cast<const uint32_t*>(&p);
             }
@@ -449,7 +443,8 @@ __global__ void __launch_bounds__(128, 1)
 // and the error word, the others give up at their next wait, in-flight loads and MMAs are
 // waited for, and the tensor memory is freed.
 // Sixteen warps in the backward epilogue, which reads, transforms, sums and stores (0.91 ms with eight for
-// 16 records of 131072 rows, the reads and stores alone 0.50), eight in the others.
+// 16 records of 131072 rows, 0.83 with sixteen, 0.72 with the derivative in packed pairs; the reads and
+// stores alone 0.50), eight in the others.
 template <int EPI> __host__ __device__ constexpr uint32_t epi_warps() { return EPI == kBackprop ? 16u : 8u; }
 template <int EPI> __host__ __device__ constexpr uint32_t epi_slices() { return epi_warps<EPI>() / 4u; }
 template <int EPI> __host__ __device__ constexpr uint32_t epi_threads() { return 64u + 32u * epi_warps<EPI>(); }
@@ -959,32 +954,6 @@ template <int KC1> constexpr size_t fsmem_bytes()
 
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// Packed FP32 pairs (sm_100 add / mul / fma .f32x2: one instruction for two lanes of work).
-__device__ __forceinline__ uint64_t pk2(float a, float b)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void upk2(uint64_t r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 // silu(a + ba), silu(b + bb) with the arithmetic of logistic() done in pairs, bit for bit: the
 // negated denominator -d = ex2 * -1 - 1 is exact, its seed 0xFEF311C0 - bits(-d) equals
 // 0x7EF311C0 - bits(d), and fma(-d, y, 1) is the same rounding as before.
