@@ -95,18 +95,19 @@ inline bool drop_convex_proven(const double c[8])
     }
     const double lip_g = 2 * l1 + l2;
     const double lip_q = 2 * r0 * l1 + 5 * l1 * l1 + 5 * l1 * l2 + r0 * (3 * l2 + l3 + l1);
-    double h = 1.0 / 64; // half-width
+    double h = 1.0 / 64; // half-width of the next interval
     for (double mu = -1.0; mu < 1.0;) { // [-1, mu] is proven
-        const double x = mu + h;
+        const double half = std::fmin(h, 0.5 * (1 - mu)); // the bounds hold within [-1, 1] only
+        const double x = mu + half;
         double rp, rpp;
         const double r = drop_radius(c, x, &rp, &rpp);
         const double s2 = 1 - x * x;
         const double g = r + x * rp;
         const double q = r * r + 2 * s2 * rp * rp - r * (s2 * rpp - x * rp);
-        if (r - l1 * h > 1e-5 && g - lip_g * h > 1e-5 && q - lip_q * h > 1e-5) {
-            mu += 2 * h;
+        if (r - l1 * half > 1e-5 && g - lip_g * half > 1e-5 && q - lip_q * half > 1e-5) {
+            mu += 2 * half;
             h = std::fmin(2 * h, 1.0 / 64);
-        } else if ((h *= 0.5) < 1e-4) {
+        } else if ((h = 0.5 * half) < 1e-4) {
             return false; // too close to the margin: the samples decide
         }
     }
