@@ -32,7 +32,6 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
-#include <cstddef>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -97,13 +96,11 @@ __device__ __forceinline__ double nan64() { return __longlong_as_double(0x7ff800
 // (s, p) of a focal record, or NaN when the record is unavailable (flags, sign, finiteness).
 __device__ __forceinline__ double2 load_sample(const icp_focal_sample* f, uint64_t i)
 {
-    // (s, p) sit 32 bytes into a 144-byte record: one aligned 16-byte load
-    const double2 sp = __ldg(reinterpret_cast<const double2*>(&f[i].intensity_s));
-    const double s = sp.x, p = sp.y;
+    // two loads: a record asks for the alignment of a double, so that the pair need not lie on 16 bytes
+    const double s = __ldg(&f[i].intensity_s), p = __ldg(&f[i].intensity_p);
     const bool good = __ldg(&f[i].flags) == 0u && s >= 0 && p >= 0 && finite64(s + p);
     return good ? make_double2(s, p) : make_double2(nan64(), nan64());
 }
-static_assert(offsetof(icp_focal_sample, intensity_s) == 32 && sizeof(icp_focal_sample) == 144, "load_sample's layout");
 __device__ __forceinline__ bool available(double2 v) { return v.x == v.x; }
 
 __device__ __forceinline__ void warp_count(uint32_t* counters, int which, bool pred)
