@@ -14,6 +14,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "icp_quot.cuh"
+
 namespace icp {
 
 constexpr double kPi = 3.141592653589793238462643383279502884;
@@ -54,33 +56,6 @@ template <class R> __device__ __forceinline__ bool finite_r(R x)
     return x == x && rabs(x) <= (sizeof(R) == 4 ? R(3.4028234663852886e38) : R(1.7976931348623157e308));
 }
 
-// Quotients by one divisor, rounded as the division operator rounds them.  The reciprocal is
-// evaluated once (correctly rounded), and each quotient is refined twice with the exact FMA
-// remainder: Markstein's theorem (IBM J. Res. Dev. 34, 1990) gives the correctly rounded quotient
-// from a correctly rounded reciprocal and a faithful quotient, away from overflow and underflow.
-// Numerators or divisors outside 2^-900 .. 2^900 take the operator (zeros keep their sign).  The
-// operator costs the FP64 trace kernels a divergent call for every zero component and the same
-// reciprocal again for every component of a vector.
-struct DivBy {
-    double b, y;
-    bool ok;
-};
-__device__ __forceinline__ bool mid_range(double x)
-{
-    return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x07b00000u < 0x70800000u;
-}
-__device__ __forceinline__ DivBy div_by(double b) { return {b, __drcp_rn(b), mid_range(b)}; }
-__device__ __forceinline__ double quot(double a, const DivBy& d)
-{
-    const double q0 = a * d.y;
-    const double q1 = fma(fma(-d.b, q0, a), d.y, q0);
-    double q = fma(fma(-d.b, q1, a), d.y, q1);
-    if (!(mid_range(a) && d.ok)) {
-        q = q0;
-        if (!(a == 0 && d.ok)) q = a / d.b;
-    }
-    return q;
-}
 __device__ __forceinline__ V3<double> quot(V3<double> a, const DivBy& d) { return {quot(a.x, d), quot(a.y, d), quot(a.z, d)}; }
 
 // Unit vector.  FP64: the reference's scale-then-normalise (math.hpp:38-47) so that exit
