@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/icp_b200.h"
+#include "../host/icp_batch_chunk.hpp"
 #include "../host/icp_drop_host.hpp"
 #include "../host/icp_host_math.hpp"
 #include "icp_internal.h"
@@ -48,14 +49,6 @@ int ok()
         const cudaError_t e_ = (call);                                                                  \
         if (e_ != cudaSuccess) return fail(ICP_ERR_DEVICE, "%s failed: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
-
-// Default ray ids per chunk: about eight chunks per resident warp, within 64..1024.  A warp drains
-// its lanes at the end of every chunk, which costs one ray's chain; a batch with fewer chunks than
-// warps leaves the chip idle, which costs more.  32 drops at 180 x 360, chains of 10 (1.6e7 rays):
-// 18.9 ms at 8192, 9.9 at 1024, 9.3 at 256; 1.1e8 rays: 57, 51 and 51 ms; 1.6e5 rays: 16.2, 3.7, 2.2 ms.
-constexpr uint32_t kChunkMin = 64u, kChunkMax = 1024u, kChunksPerWarp = 8u;
-// what icp_drop_batch_autotune starts from
-constexpr uint32_t kTunedChunk = 8192u;
 
 icp_drop_record record_of(const icp_drop_item& it, const icp_batch_settings& s)
 {
@@ -104,10 +97,7 @@ int launch_shape(icp_context* c, const icp_batch_settings& s, uint64_t rays, Sha
     if (per_sm <= 0) return fail(ICP_ERR_DEVICE, "batch trace kernel cannot be resident");
     if (s.blocks_per_sm) per_sm = std::min<int>(per_sm, (int)s.blocks_per_sm);
     sh.blocks = (uint32_t)per_sm * (uint32_t)c->sms;
-    if (!sh.chunk) {
-        const uint64_t warps = (uint64_t)sh.blocks * (sh.threads / 32u);
-        sh.chunk = (uint32_t)std::min<uint64_t>(kChunkMax, std::max<uint64_t>(kChunkMin, rays / (warps * kChunksPerWarp)));
-    }
+    sh.chunk = H::batch_chunk(sh.chunk, rays, (uint64_t)sh.blocks * (sh.threads / 32u));
     // a warp flushes its lanes' 32-bit counters once per chunk: keep a chunk within their range
     sh.chunk = (uint32_t)std::max<uint64_t>(32u, std::min<uint64_t>(sh.chunk, lane_rays_max(s.max_internal_hits)));
     return ICP_OK;
@@ -470,17 +460,25 @@ extern "C" int icp_drop_batch_autotune(icp_context* c, const icp_drop_item* item
         it.rays = std::min<uint64_t>(it.rays, 1ull << 21);
         rays += it.rays;
     }
+    // Chunks come out no larger than the ray count allows (batch_chunk): sizes that come to the same one
+    // are timed once.  The default's own size is among them, and another has to be 2 % faster.
     static const uint32_t kThreads[] = {128u, 256u};
-    static const uint32_t kChunks[] = {2048u, 8192u, 32768u};
-    double best = 0;
-    uint32_t best_t = 256u, best_c = kTunedChunk;
-    for (uint32_t t : kThreads)
+    static const uint32_t kChunks[] = {2048u, 8192u, 32768u, H::kChunkMax};
+    double best = 0, best_merit = 0;
+    uint32_t best_t = 256u, best_c = H::kChunkMax, stored_c = 0u;
+    for (uint32_t t : kThreads) {
+        icp_batch_settings s = *settings;
+        s.block_threads = t;
+        s.chunk_rays = H::kChunkMax;
+        Shape sh;
+        if (launch_shape(c, s, rays, sh)) continue;
+        const uint32_t by_count = sh.chunk;
+        std::vector<uint32_t> timed;
         for (uint32_t ch : kChunks) {
-            icp_batch_settings s = *settings;
-            s.block_threads = t;
             s.chunk_rays = ch;
-            Shape sh;
             if (launch_shape(c, s, rays, sh)) continue;
+            if (std::find(timed.begin(), timed.end(), sh.chunk) != timed.end()) continue;
+            timed.push_back(sh.chunk);
             if (const int e = prepare(c, n, s)) return e;
             std::vector<double> w;
             double secs = 1e30;
@@ -493,18 +491,21 @@ extern "C" int icp_drop_batch_autotune(icp_context* c, const icp_drop_item* item
                 cudaEventElapsedTime(&ms, c->ev0, c->ev1);
                 secs = ms * 1e-3;
             }
-            const double rate = double(rays) / secs;
-            if (rate > best) {
+            const double rate = double(rays) / secs, merit = sh.chunk == by_count ? 1.02 * rate : rate;
+            if (merit > best_merit) {
+                best_merit = merit;
                 best = rate;
                 best_t = t;
                 best_c = ch;
+                stored_c = sh.chunk == by_count ? 0u : ch;
             }
         }
+    }
     auto& tuned = c->batch.tuned;
     tuned.erase(std::remove_if(tuned.begin(), tuned.end(),
                                [&](const BatchState::Tuned& x) { return x.precision == settings->precision && x.nt == settings->nt; }),
                 tuned.end());
-    tuned.push_back({settings->precision, settings->nt, best_t, best_c});
+    tuned.push_back({settings->precision, settings->nt, best_t, stored_c});
     settings->block_threads = best_t;
     settings->chunk_rays = best_c;
     if (best_rays_per_second) *best_rays_per_second = best;

@@ -384,7 +384,8 @@ typedef struct {
     icp_cdf_policy policy;
     uint32_t block_threads;   /* 0: autotuned or 256                                        */
     uint32_t blocks_per_sm;   /* 0: as many as fit                                          */
-    uint32_t chunk_rays;      /* ray ids per work-queue chunk, 0: autotuned or by ray count */
+    uint32_t chunk_rays;      /* most ray ids per work-queue chunk (fewer where a warp would
+                                 get fewer than eight chunks), 0: autotuned or by ray count */
     uint32_t use_graph;       /* 1: launch the batch as a captured CUDA graph (replayed when
                                  the next batch has the same shape)                         */
 } icp_batch_settings;
