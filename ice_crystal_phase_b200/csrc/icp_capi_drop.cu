@@ -219,10 +219,15 @@ HexLaunch drop_launch(const icp_drop_record* r, const icp_grid* g, const double*
 
 // Drop exits spread continuously over the sphere, so a shared table of a few thousand cells
 // saturates within one block and only adds probes: by default exits go straight to the FP64
-// histogram (fire-and-forget L2 reductions).  A table can still be requested.
-int table_slots(const icp_tuning& t, uint32_t& slots)
+// histogram (fire-and-forget L2 reductions).  On a coarse grid those collide, and a table holds
+// the whole grid with a quarter of its slots to spare: 3e7 rays of the oblate drop take 60 / 49 / 16.3 / 12.2 ms
+// straight and 10.2 / 10.3 / 10.2 / 11.6 with the table at 64 / 192 / 1152 / 1568 cells, 10.0 and 12.2 at
+// 2048; 1e6 FP64 rays 2.50 / 2.11 / 1.76 and 1.79 / 1.79 / 1.78 at 64 / 192 / 1152, where the table is no
+// faster.  A table can be requested, or refused, for any grid.
+constexpr uint32_t kTableSlots = 2048u, kTableCells32 = 1536u, kTableCells64 = 512u;
+int table_slots(const icp_tuning& t, uint64_t cells, bool f32, uint32_t& slots)
 {
-    slots = 0u;
+    slots = cells <= (f32 ? kTableCells32 : kTableCells64) ? kTableSlots : 0u;
     if (t.hash_slots) slots = t.hash_slots == 1 ? 0u : t.hash_slots;
     if (slots & (slots - 1)) return fail(ICP_ERR_INVALID_ARGUMENT, "hash_slots must be a power of two");
     return ICP_OK;
@@ -238,7 +243,7 @@ int drop_trace_enqueue(icp_context* c, const icp_drop_record* r, uint64_t first,
     if (threads < 64 || threads > max_threads || threads % 32)
         return fail(ICP_ERR_INVALID_ARGUMENT, "block_threads must be 64..%u, multiple of 32", max_threads);
     uint32_t slots;
-    if (const int e = table_slots(r->tuning, slots)) return e;
+    if (const int e = table_slots(r->tuning, (uint64_t)g->nt * g->np, f32, slots)) return e;
     int per_sm = f32 ? drop_blocks_per_sm_f32(slots, g->nt, threads) : drop_blocks_per_sm_f64(slots, g->nt, threads);
     if (per_sm <= 0) return fail(ICP_ERR_DEVICE, "drop trace kernel cannot be resident");
     if (r->tuning.blocks_per_sm) per_sm = std::min<int>(per_sm, (int)r->tuning.blocks_per_sm);

@@ -246,7 +246,7 @@ void drop_bounds(const double c[8], double& r_center, double& r_out);
 int validate_record(const icp_drop_record* r);
 int validate_grid(const icp_drop_record* r);
 int grid_of(const icp_drop_record* r, icp_grid& g);
-int table_slots(const icp_tuning& t, uint32_t& slots);
+int table_slots(const icp_tuning& t, uint64_t cells, bool f32, uint32_t& slots);
 HexLaunch drop_launch(const icp_drop_record* r, const icp_grid* g, const double* d_edges, const float* edges_f,
                       double* d_mass, void* d_stats, double area_weight, uint32_t slots);
 int finish_report(const icp_drop_record* r, const unsigned char* raw_stats, const CdfDeviceReport& cdf, double power,
