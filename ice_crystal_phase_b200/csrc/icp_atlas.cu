@@ -961,10 +961,15 @@ int icp_atlas_compose(icp_context* ctx, uint32_t nodes, uint32_t nt, uint32_t np
     };
     // K = 9 keeps the most warps per row that the loads still serve twice (28 nodes at 900 x 1800: 1.60 ms
     // a record, 1.76 with K = 15, 1.93 with K = 19); rows beyond 256 threads of 9 need 17, and fewer
-    // rows than two per SM take 5 for the warps
+    // rows than two per SM take 5 for the warps.  A row of 256 cells or fewer waits for its entries one after
+    // the other and wants four warps: one cell a thread (28 nodes at 60 x 120 80 us, 157 with K = 5; 127 x 254
+    // 93 and 171), or three where rows fill the chip (900 x 180: 163, 211 with one, 226 with nine)
+    const uint32_t sms = (uint32_t)ctx->sms;
     cudaError_t e;
     if (np > 9u * 256u) e = run(atlas_compose_kernel<17>, 17u);
-    else if (nt < 2u * (uint32_t)ctx->sms && np <= 5u * 256u) e = run(atlas_compose_kernel<5>, 5u);
+    else if (np <= 256u && (nt < 3u * sms || np <= 128u)) e = run(atlas_compose_kernel<1>, 1u);
+    else if (np <= 256u) e = run(atlas_compose_kernel<3>, 3u);
+    else if (nt < 2u * sms && np <= 5u * 256u) e = run(atlas_compose_kernel<5>, 5u);
     else e = run(atlas_compose_kernel<9>, 9u);
     ICP_CUDA(e);
     count_launch();
