@@ -42,6 +42,7 @@
 
 #include "../../include/icp_b200.h"
 #include "icp_internal.h"
+#include "icp_outward.cuh"
 
 using namespace icp;
 
@@ -87,15 +88,6 @@ template <class T> __host__ __device__ __forceinline__ T root(T x)
     if constexpr (std::is_same_v<T, float>) return sqrtf(x);
     else return sqrt(x);
 }
-// nextUp: the least representable number above x (+inf and NaN unchanged, either zero to the
-// least positive subnormal); nextDown(x) = -nextUp(-x).  x plus the least subnormal, rounded up, is
-// that number for every x but -inf (checked over all 2^32 binary32 values): one addition where the
-// step on the bits took six operations, and an enclosure is made of little else.  An enclosure
-// whose finite end has overflowed stays infinite, on the side that excludes it already.
-__device__ __forceinline__ float next_up(float x) { return __fadd_ru(x, 0x1p-149f); }
-__device__ __forceinline__ double next_up(double x) { return __dadd_ru(x, 0x1p-1074); }
-__device__ __forceinline__ float next_down(float x) { return __fadd_rd(x, -0x1p-149f); }
-__device__ __forceinline__ double next_down(double x) { return __dadd_rd(x, -0x1p-1074); }
 template <class T> __device__ __forceinline__ T lesser(T a, T b) { return a < b ? a : b; }
 template <class T> __device__ __forceinline__ T greater(T a, T b) { return a > b ? a : b; }
 // The same for products that are stepped outward next (which leaves no sign to a zero) and are NaN
