@@ -73,11 +73,6 @@ template <bool kFmaRcp> __device__ __forceinline__ float silu(float z)
 {
     return z * (kFmaRcp ? logistic(z) : logistic_mufu(z));
 }
-template <bool kFmaRcp> __device__ __forceinline__ float silu_grad(float z)
-{
-    const float s = kFmaRcp ? logistic(z) : logistic_mufu(z);
-    return s * (1.0f + z * (1.0f - s));
-}
 
 // Column sums of a warp's 32 x 32 block (lane = row, v[i] = column i): a butterfly
 // reduce-scatter in 31 shuffles, after which lane L holds the sum of column L in v[0].
@@ -96,8 +91,8 @@ __device__ __forceinline__ float warp_column_sum(float (&v)[32], uint32_t lane)
     return v[0];
 }
 
-// A warp's tile of 32 rows x 64 BF16 columns between its row-per-lane form (lane = row, w[32] its 64
-// values) and global memory, through 4 KB of shared memory with the 16-byte chunks of row r
+// A warp's tile of 32 rows x 64 BF16 columns from its row-per-lane form (lane = row, w[32] its 64
+// values) to global memory, through 4 KB of shared memory with the 16-byte chunks of row r
 // exchanged by r mod 8 (no bank conflicts either way): every global access then covers four whole
 // 128-byte lines, where a row per lane touches 32 half-used sectors (with the column-major copies
 // that the weight gradients read before: 1.92 ms per hidden layer of 16 records, 0.52 .. 0.60 now).
@@ -117,28 +112,6 @@ __device__ __forceinline__ void store_tile(__nv_bfloat16* dst, uint32_t ld, cons
     for (uint32_t i = 0; i < 8; ++i) {
         const uint32_t row = 4u * i + (lane >> 3), ch = lane & 7u;
         *reinterpret_cast<uint4*>(dst + (size_t)row * ld + 8u * ch) = *tile_chunk(buf, row, ch);
-    }
-    __syncwarp();
-}
-// This lane's share of a tile (issued early; the values land in `part`), then the row-per-lane form.
-__device__ __forceinline__ void load_tile(const __nv_bfloat16* src, uint32_t ld, uint32_t lane, uint4 (&part)[8])
-{
-#pragma unroll
-    for (uint32_t i = 0; i < 8; ++i)
-        part[i] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(4u * i + (lane >> 3)) * ld + 8u * (lane & 7u)));
-}
-__device__ __forceinline__ void tile_rows(const uint4 (&part)[8], uint8_t* buf, uint32_t lane, uint32_t (&w)[32])
-{
-#pragma unroll
-    for (uint32_t i = 0; i < 8; ++i) *tile_chunk(buf, 4u * i + (lane >> 3), lane & 7u) = part[i];
-    __syncwarp();
-#pragma unroll
-    for (uint32_t ch = 0; ch < 8; ++ch) {
-        const uint4 u = *tile_chunk(buf, lane, ch);
-        w[4 * ch] = u.x;
-        w[4 * ch + 1] = u.y;
-        w[4 * ch + 2] = u.z;
-        w[4 * ch + 3] = u.w;
     }
     __syncwarp();
 }
@@ -236,14 +209,14 @@ __device__ __forceinline__ void epilogue_f32(const GemmArgs& g, uint32_t taddr, 
 
 // Columns [c0, c1) (a multiple of 64) of a warp's 32 rows m0 .. m0 + 31 of a 128 x N accumulator tile
 // through a layer's epilogue: this thread's TMEM lane starts at taddr (column 0), its row is m0 + lane;
-// bias / head_w point at N values (16-byte aligned); colsum collects the bias gradient and z holds
-// the first 64 columns of z_prev already requested with load_tile (kBackprop); buf is the warp's tile
-// buffer.  Returns the partial head sum of these columns (kHead).
+// bias / head_w point at N values (16-byte aligned); buf is the warp's tile buffer.  Returns the partial
+// head sum of these columns (kHead).
 template <int N, int EPI>
 __device__ __forceinline__ float epilogue_layer(const GemmArgs& g, uint32_t taddr, uint32_t m0, uint32_t lane,
                                                 uint32_t c0, uint32_t c1, const float* bias, const float* head_w,
-                                                float* colsum, uint4 (&z)[8], uint8_t* buf)
+                                                uint8_t* buf)
 {
+    static_assert(EPI != kBackprop && EPI != kStoreF32 && EPI != kAtomicF32, "these have epilogues of their own");
     constexpr bool kHeadEpi = EPI == kHead || EPI == kHeadTrain;
     constexpr bool kTrain = EPI == kHiddenTrain || EPI == kHeadTrain;
     float yacc = 0.0f;
@@ -252,56 +225,39 @@ __device__ __forceinline__ float epilogue_layer(const GemmArgs& g, uint32_t tadd
         float v[2][32];
         umma::tmem_ld32x2(taddr + c, v[0], v[1]); // both loads in flight, one wait
         uint32_t w[32];
-        if constexpr (EPI == kBackprop) {
-            tile_rows(z, buf, lane, w);
-            if (c + 64u < c1) load_tile(g.z_prev + (size_t)m0 * N + c + 64u, N, lane, z);
+        const float4* b4 = reinterpret_cast<const float4*>(bias + c);
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+        for (int q = 0; q < 16; ++q) {
+            const float4 b = b4[q];
+            float* x = &v[q / 8][4 * (q % 8)];
+            x[0] += b.x;
+            x[1] += b.y;
+            x[2] += b.z;
+            x[3] += b.w;
+        }
+        if constexpr (kTrain)
+            if (g.out_z) {
+                pack_bf16(v, w);
+                store_tile(g.out_z + (size_t)m0 * N + c, N, w, buf, lane);
+            }
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[16 * h + i]));
-                    v[h][2 * i] *= silu_grad<false>(f.x);
-                    v[h][2 * i + 1] *= silu_grad<false>(f.y);
-                }
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[h][i] = silu<!kTrain>(v[h][i]);
+        if (g.out_h) {
             pack_bf16(v, w);
-            store_tile(g.out_dz + (size_t)m0 * N + c, N, w, buf, lane);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) atomicAdd(&colsum[c + 32u * h + lane], warp_column_sum(v[h], lane));
-        } else {
-            const float4* b4 = reinterpret_cast<const float4*>(bias + c);
+            store_tile(g.out_h + (size_t)m0 * N + c, N, w, buf, lane);
+        }
+        if constexpr (kHeadEpi) {
+            const float4* w4 = reinterpret_cast<const float4*>(head_w + c);
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
-                const float4 b = b4[q];
-                float* x = &v[q / 8][4 * (q % 8)];
-                x[0] += b.x;
-                x[1] += b.y;
-                x[2] += b.z;
-                x[3] += b.w;
-            }
-            if constexpr (kTrain)
-                if (g.out_z) {
-                    pack_bf16(v, w);
-                    store_tile(g.out_z + (size_t)m0 * N + c, N, w, buf, lane);
-                }
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[h][i] = silu<!kTrain>(v[h][i]);
-            if (g.out_h) {
-                pack_bf16(v, w);
-                store_tile(g.out_h + (size_t)m0 * N + c, N, w, buf, lane);
-            }
-            if constexpr (kHeadEpi) {
-                const float4* w4 = reinterpret_cast<const float4*>(head_w + c);
-#pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                    const float4 hw = w4[q];
-                    const float* x = &v[q / 8][4 * (q % 8)];
-                    yacc = fmaf(x[0], hw.x, yacc);
-                    yacc = fmaf(x[1], hw.y, yacc);
-                    yacc = fmaf(x[2], hw.z, yacc);
-                    yacc = fmaf(x[3], hw.w, yacc);
-                }
+                const float4 hw = w4[q];
+                const float* x = &v[q / 8][4 * (q % 8)];
+                yacc = fmaf(x[0], hw.x, yacc);
+                yacc = fmaf(x[1], hw.y, yacc);
+                yacc = fmaf(x[2], hw.z, yacc);
+                yacc = fmaf(x[3], hw.w, yacc);
             }
         }
     }
@@ -606,7 +562,7 @@ __global__ void __launch_bounds__(epi_threads<EPI>(), 1)
 #pragma unroll 1
         for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
             const uint32_t b = i & 1u;
-            uint4 z[EPI == kBackprop ? 4 : 8]; // requested before the accumulator is waited for
+            uint4 z[4]; // kBackprop: requested before the accumulator is waited for
             if constexpr (EPI == kBackprop) load_half_tile(g.z_prev + (size_t)(t * 128u + 32u * q) * N + c0, N, lane, z);
             const bool mine = live && umma::mbar_wait(&acc_full[b], (i >> 1) & 1u, kWaitLimit);
             if (!__all_sync(0xffffffffu, mine && !*abort_flag)) {
@@ -624,8 +580,7 @@ __global__ void __launch_bounds__(epi_threads<EPI>(), 1)
                 else if constexpr (EPI == kBackprop)
                     epilogue_backprop<N>(g, taddr, t * 128u + 32u * q, lane, c0, c0 + W, colsum, z, buf);
                 else
-                    y = epilogue_layer<N, EPI>(g, taddr, t * 128u + 32u * q, lane, c0, c0 + W, sbias, shead, colsum, z,
-                                               buf);
+                    y = epilogue_layer<N, EPI>(g, taddr, t * 128u + 32u * q, lane, c0, c0 + W, sbias, shead, buf);
                 umma::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) umma::mbar_arrive(&acc_empty[b]);
