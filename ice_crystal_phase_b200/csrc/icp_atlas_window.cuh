@@ -1,6 +1,7 @@
-// icp_atlas_window.cuh -- phi-index arithmetic of the cyclic composition (atlas_compose_kernel):
-// the cell of row m that output cell p reads at shift s is m = (p - s) mod np, reflected to
-// np - 1 - m for the mirrored parity; no integer division in the inner loop.  Host and device
+// icp_atlas_window.cuh -- phi-index arithmetic of the cyclic composition: the cell of a row that
+// output cell p reads at shift s is m = (p - s) mod np, reflected to np - 1 - m for the mirrored
+// parity.  atlas_compose_kernel reflects with phi_cell when it lays a row out twice and then reads plain
+// offsets; phi_sub, phi_add and phi_prev state the rule cell by cell for the host test.  Host and device
 // code alike (the host test compiles it with g++).
 #pragma once
 #include <cstdint>

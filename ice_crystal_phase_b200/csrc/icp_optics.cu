@@ -1060,9 +1060,9 @@ __global__ void __launch_bounds__(kFoldThreads) fold_slot_kernel(const icp_outgo
         if (flag) list[slot] = i;
     }
 }
-// one thread per record: the quadrature's panel count varies, so the records are dense and
-// the launch covers only them.  acc: [0] prepared, [1] unresolved, [2] branches, [3] focal-
-// pending branches, [4] largest estimated error (bits of a non-negative double)
+// A warp per record: the quadrature's panel count varies, so the records are dense and the launch
+// covers only them.  acc: [0] prepared, [1] unresolved, [2] branches, [3] focal-
+// pending branches, [4] largest estimated error (bits of a non-negative double).
 // A thousand candidates or so lie along the caustics of a 513 x 513 lattice: one thread each kept 18
 // blocks busy for 0.39 ms, a serial chain of some thousand quadrature points with a root and two quotients
 // in each.  A warp each: 0.05 ms.

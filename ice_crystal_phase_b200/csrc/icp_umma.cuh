@@ -1,8 +1,8 @@
 // icp_umma.cuh -- 5th-generation tensor-core building blocks for sm_100a, as inline PTX:
 // tensor-memory allocation, tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, one CTA), commit to an
 // mbarrier, tcgen05.ld of the accumulator, mbarriers with bounded waits, and 2-D TMA tile loads
-// (no multicast).  Operand tiles are K-major with the 128-byte swizzle that a TMA load with
-// CU_TENSOR_MAP_SWIZZLE_128B writes: row r of a tile at byte 128 r, its 16-byte chunks permuted
+// (no multicast).  Operand tiles are K-major, or MN-major where the contraction runs over the rows
+// (smem_desc_sw128_mn), with the 128-byte swizzle that a TMA load with CU_TENSOR_MAP_SWIZZLE_128B writes: row r of a tile at byte 128 r, its 16-byte chunks permuted
 // by r mod 8, 8-row groups 1024 bytes apart (tiles 1024-byte aligned).
 //
 // Shared-memory matrix descriptor (64 bit): start address >> 4 in bits [0,14), leading-dimension

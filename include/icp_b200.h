@@ -138,10 +138,11 @@ typedef struct {
 
 /* Histogram privatisation / launch tuning (all zero = autotuned defaults). */
 typedef struct {
-    uint32_t block_threads;  /* 0 = the kernel's size (FP32 drop 128, others 256), else 64 up
-                              * to that size, a multiple of 32                               */
+    uint32_t block_threads;  /* 0 = the kernel's size (drops 128, prisms 256), else a multiple
+                              * of 32 from 64 to 256 (FP32 drop: to 128)                     */
     uint32_t blocks_per_sm;  /* resident blocks per SM requested                              */
-    uint32_t hash_slots;     /* shared-memory table slots (power of two; 0 = default; 1 = off) */
+    uint32_t hash_slots;     /* shared-memory table slots (power of two; 0 = default: prisms 4096,
+                              * drops 2048 on coarse grids and none on others; 1 = off)     */
     uint32_t reserved;
 } icp_tuning;
 
