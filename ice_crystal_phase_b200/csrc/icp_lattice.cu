@@ -623,8 +623,8 @@ struct BlockTally {
     unsigned long long first_problem;
 };
 
-// What bounds it: instruction supply and the dependent chains of the interval enclosures (a quarter of
-// the issue slots; no memory traffic to speak of), with half of the lanes waiting for the warp's longest
+// What bounds it: instruction supply and the dependent chains of the interval enclosures (half of
+// the issue slots; no memory traffic to speak of), with a third of the lanes waiting for the warp's longest
 // search.  Figures for 513 x 513 rays, 6.3 ms with the solver inlined for the entry and again for the
 // internal encounters: one copy of it in one loop 2.2 ms, outward steps of one instruction 1.3 ms, one
 // enclosure a step and one exit before the refinement 0.91 ms.  Four blocks per SM (128 registers, a few
