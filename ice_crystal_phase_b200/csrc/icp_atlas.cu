@@ -650,6 +650,68 @@ __global__ void __launch_bounds__(256) atlas_compose_kernel(const double* __rest
     for (uint32_t p = threadIdx.x; p < np; p += blockDim.x) out[(uint64_t)t * np + p] = row[p];
 }
 
+// The same for rows of at most kNarrow cells: a thread per cell, so that a row has a warp on each
+// quarter of its SM, and the next coupling row's cells and entries on their way while this one's are
+// added.  Bound by the chain of dependent additions, one per weight.  28 nodes at 60 x 120 (1920 weights):
+// 157 us with five cells a thread, whose one warp also waits for its own products, 80 with one,
+// 77 with the loads ahead; 12 nodes at 60 x 117 67, 41 and 38 us.
+constexpr uint32_t kNarrow = 256;
+__global__ void __launch_bounds__(kNarrow) atlas_compose_narrow_kernel(const double* __restrict__ mass,
+                                                                       const uint32_t* __restrict__ counts,
+                                                                       const uint32_t* __restrict__ shifts,
+                                                                       const double2* __restrict__ values, uint32_t nodes,
+                                                                       uint32_t nt, uint32_t np, double* __restrict__ out)
+{
+    __shared__ double row[compose_cells(kNarrow, kNarrow, 1)]; // as above
+    __shared__ double2 s_w[kNarrow / 2]; // an entry covers two shifts, or is followed by a zero weight
+    __shared__ uint32_t s_from[kNarrow / 2];
+    const uint32_t t = blockIdx.x, x = threadIdx.x, cells = compose_cells(np, blockDim.x, 1);
+    const uint64_t rows = (uint64_t)nodes * 2;
+    uint64_t r = 0;
+    uint32_t cnt = 0, ahead = counts[0]; // entries of rows r and r + 1
+    double v = 0.0;
+    double2 w = make_double2(0.0, 0.0);
+    uint32_t from = 0;
+    // this thread's cell and entry of the next row that has entries, from row `at` on
+    auto fetch = [&](uint64_t at) {
+        cnt = ahead;
+        while (!cnt && ++at < rows) cnt = counts[at];
+        ahead = at + 1u < rows ? counts[at + 1u] : 0u;
+        if (cnt) {
+            if (x < np) v = mass[((at >> 1) * nt + t) * np + x];
+            if (x < cnt) {
+                w = values[at * np + x];
+                from = np - 1u - shifts[at * np + x];
+            }
+        }
+        return at;
+    };
+    double acc = 0.0;
+    r = fetch(0);
+    while (cnt) {
+        __syncthreads(); // the previous row and entries are no longer read
+        if (x < np)
+            for (uint32_t c = phi_cell(x, np, (int)(r & 1u)); c < cells; c += np) row[c] = v;
+        if (x < cnt) {
+            s_w[x] = w;
+            s_from[x] = from;
+        }
+        const uint32_t entries = cnt;
+        __syncthreads();
+        if (r + 1u < rows) r = fetch(r + 1u);
+        else cnt = 0;
+#pragma unroll 4
+        for (uint32_t e = 0; e < entries; ++e) {
+            const double2 we = s_w[e];
+            const double* at = row + (s_from[e] + x); // cell x - s - 1
+            acc = acc + we.x * at[1];
+            const double both = acc + we.y * at[0];
+            acc = we.y != 0.0 ? both : acc;
+        }
+    }
+    if (x < np) out[(uint64_t)t * np + x] = acc;
+}
+
 int validate_settings(const icp_atlas_settings* s)
 {
     if (!s) return fail(ICP_ERR_INVALID_ARGUMENT, "icp_atlas: null settings");
@@ -961,15 +1023,18 @@ int icp_atlas_compose(icp_context* ctx, uint32_t nodes, uint32_t nt, uint32_t np
     };
     // K = 9 keeps the most warps per row that the loads still serve twice (28 nodes at 900 x 1800: 1.60 ms
     // a record, 1.76 with K = 15, 1.93 with K = 19); rows beyond 256 threads of 9 need 17, and fewer
-    // rows than two per SM take 5 for the warps.  A row of 256 cells or fewer waits for its entries one after
-    // the other and wants four warps: one cell a thread (28 nodes at 60 x 120 80 us, 157 with K = 5; 127 x 254
-    // 93 and 171), or three where rows fill the chip (900 x 180: 163, 211 with one, 226 with nine)
+    // rows than two per SM take 5 for the warps.  Rows of kNarrow cells and fewer have a kernel of their
+    // own (127 x 254 89 us, 171 with K = 5), but for many rows of more than half as many cells, where K = 3 serves
+    // the loads better (900 x 180 163 us, 213 with the narrow kernel, 226 with K = 9; 320 x 250 153 and 131)
     const uint32_t sms = (uint32_t)ctx->sms;
     cudaError_t e;
     if (np > 9u * 256u) e = run(atlas_compose_kernel<17>, 17u);
-    else if (np <= 256u && (nt < 3u * sms || np <= 128u)) e = run(atlas_compose_kernel<1>, 1u);
-    else if (np <= 256u) e = run(atlas_compose_kernel<3>, 3u);
-    else if (nt < 2u * sms && np <= 5u * 256u) e = run(atlas_compose_kernel<5>, 5u);
+    else if (np <= kNarrow && np > kNarrow / 2u && nt >= 4u * sms) e = run(atlas_compose_kernel<3>, 3u);
+    else if (np <= kNarrow) {
+        atlas_compose_narrow_kernel<<<nt, (np + 31u) / 32u * 32u, 0, ctx->stream>>>(d_mass, counts, shifts, values, nodes,
+                                                                                  nt, np, d_out);
+        e = cudaGetLastError();
+    } else if (nt < 2u * sms && np <= 5u * 256u) e = run(atlas_compose_kernel<5>, 5u);
     else e = run(atlas_compose_kernel<9>, 9u);
     ICP_CUDA(e);
     count_launch();
