@@ -186,23 +186,27 @@ __device__ __forceinline__ void epilogue_backprop(const GemmArgs& g, uint32_t ta
     }
 }
 
-// Columns [0, N) of one row of a 128 x N accumulator tile to FP32 (kStoreF32, kAtomicF32): this
-// thread's TMEM lane starts at taddr, m is the output row.
+// Columns [c0, c1) (a multiple of 64) of one row of a 128 x N accumulator tile to FP32 (kStoreF32,
+// kAtomicF32): this thread's TMEM lane starts at taddr, m is the output row.  Both loads of 64 columns are
+// in flight together (256 x 128 x 131072 in 148 splits: 138 us so, 148 one after the other).
 template <int EPI>
 __device__ __forceinline__ void epilogue_f32(const GemmArgs& g, uint32_t taddr, uint32_t m, uint32_t c0, uint32_t c1)
 {
 #pragma unroll 1
-    for (uint32_t c = c0; c < c1; c += 32u) {
-        float v[32];
-        umma::tmem_ld32(taddr + c, v);
-        if constexpr (EPI == kStoreF32) {
-            float4* d = reinterpret_cast<float4*>(g.out_f32 + (size_t)m * g.ld_out + c);
+    for (uint32_t c = c0; c < c1; c += 64u) {
+        float v[2][32];
+        umma::tmem_ld32x2(taddr + c, v[0], v[1]);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) d[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        } else {
-            float* d = g.out_f32 + (size_t)m * g.ld_out + c;
+        for (int h = 0; h < 2; ++h) {
+            float* out = g.out_f32 + (size_t)m * g.ld_out + c + 32u * h;
+            if constexpr (EPI == kStoreF32) {
+                float4* d = reinterpret_cast<float4*>(out);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) atomicAdd(d + i, v[i]);
+                for (int q = 0; q < 8; ++q) d[q] = make_float4(v[h][4 * q], v[h][4 * q + 1], v[h][4 * q + 2], v[h][4 * q + 3]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) atomicAdd(out + i, v[h][i]);
+            }
         }
     }
 }
